@@ -1,0 +1,115 @@
+"""The FP64 entry points of the C ABI at the sizes where their work splits change: block and warp edges, remainders,
+the smallest and largest grids. Each against plain NumPy / torch FP64 of the same quantity."""
+
+import ctypes as C
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+def _abi():
+    import torch
+
+    from devinproj_b200 import _lib
+    from devinproj_b200.device import stream_handle
+    return torch, _lib.lib(), stream_handle()
+
+
+def _grid(L, box, rc, pos=None):
+    from devinproj_b200 import _lib
+    g = _lib.AcsGrid()
+    if box is None:
+        lo, hi = (np.ascontiguousarray(x) for x in (np.nanmin(pos, 0), np.nanmax(pos, 0)))
+        assert L.acs_grid_setup(C.byref(g), None, 0, lo.ctypes.data, hi.ctypes.data, float(rc)) == 0
+    else:
+        b = np.ascontiguousarray(box, dtype=float)
+        assert L.acs_grid_setup(C.byref(g), b.ctypes.data, 1, None, None, float(rc)) == 0
+    g.rc2 = rc ** 2
+    return g
+
+
+def _reference_lists(pos, g):
+    """Every atom's neighbours by the reference's binning, stencil and FP64 filter (accusim/forces.py:279-321), in
+    stencil order and ascending index within a cell."""
+    nc, lo, span = np.array(g.ncell), np.array(g.lo), np.array(g.span)
+    with np.errstate(invalid="ignore"):
+        t = (pos - lo) / span * nc
+        cell = np.where(t >= 1, np.where(t >= nc - 1, nc - 1, np.floor(np.where(np.isfinite(t), t, 0))), 0).astype(int)
+    out = []
+    for i in range(len(pos)):
+        d = cell - cell[i]
+        if g.periodic:
+            d = np.where(nc >= 3, (d + 1) % nc - 1, d)
+        near = np.all(np.abs(d) <= 1, axis=1)
+        near[i] = False
+        j = np.flatnonzero(near)
+        with np.errstate(invalid="ignore", over="ignore"):
+            r = pos[j] - pos[i]
+            if g.periodic:
+                b = np.array(g.box)
+                r = r - b * np.round(r / b)
+            close = (r[:, 0] * r[:, 0] + r[:, 1] * r[:, 1]) + r[:, 2] * r[:, 2] < g.rc2
+        j = j[close]
+        rank = (d[j] + 1) @ np.array([9, 3, 1])
+        out.append(j[np.lexsort((j, rank))])
+    return out
+
+
+# (cells per axis, atoms, periodic): one cell, the image found per pair (3 cells), stencil images (4 and more), a warp
+# per cell (1024 cells and more) with ragged and with crowded cells, open boxes
+LIST_FORMS = [((1, 1, 1), 70, True), ((3, 3, 3), 500, True), ((4, 3, 7), 900, True), ((4, 4, 5), 33, True),
+              ((5, 4, 6), 1300, True), ((11, 10, 10), 4500, True), ((4, 16, 17), 4400, True), ((12, 11, 9), 4800, False),
+              ((2, 2, 3), 400, False)]
+
+
+@pytest.mark.parametrize("cells,n,periodic", LIST_FORMS)
+@pytest.mark.parametrize("kind", ["inside", "edges", "outside", "clustered"])
+@pytest.mark.parametrize("unit", [1.0, 1e-30])
+def test_list_is_the_reference_filter_entry_by_entry(cells, n, periodic, kind, unit):
+    """Whole lists, in order, for positions inside the box, on cell and box edges, outside it (a caller's unwrapped atoms,
+    a NaN, an infinity) and crowded into a few cells; in a unit whose squares underflow FP32 too. Exact."""
+    torch, L, st = _abi()
+    rng = np.random.default_rng(n)
+    rc = 1.1 * unit
+    box = (np.array(cells) + rng.uniform(0.02, 0.9, 3) * (np.array(cells) > 1)) * rc
+    if cells == (1, 1, 1):
+        box = np.array([1.3, 2.2, 2.9]) * rc
+    pos = rng.uniform(0, 1, (n, 3)) * box
+    if kind == "edges":
+        k = rng.integers(0, 3 * n, n)
+        edge = rng.integers(0, np.array(cells) + 1, (n, 3)) / np.array(cells) * box
+        pos.reshape(-1)[k] = np.nextafter(edge.reshape(-1)[k], rng.choice([-1e9, 1e9], n) * unit)
+        pos[:15] = pos[15:30] + rc * np.array([1.0, 0, 0])   # r^2 next to rc^2
+        if periodic:
+            pos = np.abs(pos)
+    elif kind == "outside":
+        far = rng.choice(n, n // 4, replace=False)
+        pos[far] += rng.integers(-2, 3, (len(far), 3)) * box
+        if periodic:
+            pos[1], pos[2] = np.nan, [np.inf, 0.1 * rc, 0.2 * rc]
+    elif kind == "clustered":
+        pos[: n // 2] = box * 0.3 + rng.normal(0, 0.3 * rc, (n // 2, 3))
+    g = _grid(L, box if periodic else None, rc, pos)
+    ref = _reference_lists(pos, g)
+    maxnb = max(max(len(r) for r in ref), 1)
+    p = torch.from_numpy(pos).cuda()
+    nbr = torch.full(((n + 31) // 32 * 32 * maxnb,), -7, dtype=torch.int32, device="cuda")
+    nnb = torch.full((n,), -7, dtype=torch.int32, device="cuda")
+    status = torch.zeros(8, dtype=torch.int32, device="cuda")
+    work = torch.empty(L.acs_nlist_work_bytes(n, C.byref(g)) + 4, dtype=torch.uint8, device="cuda")
+    assert L.acs_nlist_build(p.data_ptr(), n, C.byref(g), maxnb, nbr.data_ptr(), nnb.data_ptr(), work.data_ptr() + 4,
+                             work.numel() - 4, status.data_ptr(), st) == 0
+    got_n = nnb.cpu().numpy()
+    assert np.array_equal(got_n, [len(r) for r in ref]) and not status.cpu().numpy()[0]
+    rows = nbr.cpu().numpy().reshape(-1, maxnb, 32)
+    for i, r in enumerate(ref):
+        assert np.array_equal(rows[i // 32, :len(r), i % 32], r)
+    # one entry too few: every count is still reported, nothing is written past the capacity
+    if maxnb > 1:
+        nbr.fill_(-7)
+        assert L.acs_nlist_build(p.data_ptr(), n, C.byref(g), maxnb - 1, nbr.data_ptr(), nnb.data_ptr(),
+                                 work.data_ptr() + 4, work.numel() - 4, status.data_ptr(), st) == 0
+        s = status.cpu().numpy()
+        assert s[0] == 1 and s[1] == maxnb and np.array_equal(nnb.cpu().numpy(), got_n)
+        assert bool((nbr[(n + 31) // 32 * 32 * (maxnb - 1):] == -7).all())
