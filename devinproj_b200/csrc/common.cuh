@@ -2,6 +2,7 @@
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <string.h>
 
 #include "accusim_b200.h"
 
@@ -34,6 +35,21 @@ __device__ __forceinline__ double min_image(double d, double box, double inv_box
   return sub(d, mul(box, k));
 }
 
+// The same, bit for bit, without the division for almost every pair. A difference below 0.49 box (compared through
+// the high words, on the integer pipe) has k = 0 and stays as it is. Otherwise t = d (1/box) differs from the IEEE
+// quotient d / box by under 3e-16 |d / box|, and rint only changes at half-integers, so rint(t) is rint(d / box)
+// unless t lies within 1e-9 of a half-integer (or |t| is huge); there the quotient decides as in the reference. rint
+// by adding and subtracting 1.5 2^52 (round to nearest even, exact for |t| < 2^51): two additions at the full FP64
+// rate, where the rint and trunc instructions run at a quarter of it or less.
+static __device__ __noinline__ double min_image_quotient(double d, double box) { return min_image(d, box); }
+__device__ __forceinline__ double image1(double d, double box, double inv_box, int near_hi) {
+  if ((__double2hiint(d) & 0x7fffffff) < near_hi) return d;
+  const double t = d * inv_box;
+  const double k0 = sub(add(t, 6755399441055744.0), 6755399441055744.0);
+  if (fabs(t - k0) < 0.5 - 1e-9 && fabs(t) < 1e6) return sub(d, mul(box, k0));
+  return min_image_quotient(d, box);   // out of line: rare, and its registers stay out of the pair loops
+}
+
 // np.einsum("ij,ij->i") over 3 components, summed left to right without FMA.
 __device__ __forceinline__ double norm2(double dx, double dy, double dz) {
   return add(add(mul(dx, dx), mul(dy, dy)), mul(dz, dz));
@@ -44,6 +60,42 @@ struct Box3 {
   double inv[3];   // 1 / L, for min_image's multiply
   int periodic;
 };
+
+// A box with the constants the pair kernels' minimum image uses; an edge that is not a positive number takes the
+// quotient everywhere.
+struct ImageBox {
+  double L[3], inv[3];
+  int near_hi[3];  // high word of 0.49 L: differences below it are their own minimum image
+  int periodic;
+};
+
+inline ImageBox image_box(const double* edges3, int periodic) {
+  ImageBox b;
+  for (int k = 0; k < 3; ++k) {
+    b.L[k] = edges3 ? edges3[k] : 0.0;
+    b.inv[k] = b.L[k] != 0.0 ? 1.0 / b.L[k] : 0.0;
+    const double near_d = b.L[k] > 0.0 && b.L[k] <= 1e300 ? 0.49 * b.L[k] : 0.0;
+    uint64_t bits;
+    memcpy(&bits, &near_d, 8);
+    b.near_hi[k] = (int)(bits >> 32);
+  }
+  b.periodic = periodic && edges3;
+  return b;
+}
+
+// Whether a difference is its own minimum image on every axis, by the high words alone.
+__device__ __forceinline__ bool near_image(double dx, double dy, double dz, const ImageBox& b) {
+  return (__double2hiint(dx) & 0x7fffffff) < b.near_hi[0] && (__double2hiint(dy) & 0x7fffffff) < b.near_hi[1] &&
+         (__double2hiint(dz) & 0x7fffffff) < b.near_hi[2];
+}
+
+__device__ __forceinline__ void image3(double& dx, double& dy, double& dz, const ImageBox& b) {
+  if (b.periodic) {
+    dx = image1(dx, b.L[0], b.inv[0], b.near_hi[0]);
+    dy = image1(dy, b.L[1], b.inv[1], b.near_hi[1]);
+    dz = image1(dz, b.L[2], b.inv[2], b.near_hi[2]);
+  }
+}
 
 __device__ __forceinline__ void min_image3(double& dx, double& dy, double& dz, const Box3& b) {
   if (b.periodic) {

@@ -8,6 +8,7 @@
 
 #include <algorithm>
 #include <mutex>
+#include <type_traits>
 
 #include "common.cuh"
 
@@ -556,43 +557,229 @@ struct DSFPar {
   double a, rc, k, c, erc, fshift, self_coef;
 };
 
-template <bool DENSE>
-__global__ void __launch_bounds__(kBlock) k_lj64(const double* __restrict__ pos, const int32_t* __restrict__ sp, int64_t n,
-                                                  Box3 box, const int32_t* __restrict__ nbr,
-                                                  const int32_t* __restrict__ nnb, int maxnb, LJTab t,
+// An atom's position and one more value (species or charge) as one 32-byte sector, read by one 256-bit load: a pair
+// loop that gathers from the caller's arrays touches up to four sectors per neighbour in four loads.
+struct __align__(32) Packed {
+  double x, y, z, w;
+};
+
+__device__ __forceinline__ Packed ld_packed(const Packed* p) {
+  Packed v;
+  asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v.x), "=d"(v.y), "=d"(v.z), "=d"(v.w) : "l"(p));
+  return v;
+}
+
+// Packs positions with the species index (sp) or the charge (q) and clears the energy reduction's ticket.
+__global__ void k_pack(const double* __restrict__ pos, const int32_t* __restrict__ sp, const double* __restrict__ q,
+                       int64_t n, Packed* __restrict__ out, unsigned int* ticket) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i == 0) *ticket = 0u;
+  if (i >= n) return;
+  Packed v;
+  v.x = pos[3 * i];
+  v.y = pos[3 * i + 1];
+  v.z = pos[3 * i + 2];
+  v.w = sp ? __hiloint2double(0, sp[i]) : q[i];
+  out[i] = v;
+}
+
+// How the pair kernels split their work: a block of 256 threads takes 256 / phases atoms, and the `phases` threads of
+// an atom (256 / phases apart in the block) share its neighbours, entry k going to phase k mod phases. Consecutive
+// threads are consecutive atoms, so a list row is read in whole sectors for every split up to 32 (8 atoms a row).
+struct PairSplit {
+  int log2_phases, atoms;   // phases = 1 << log2_phases, atoms = 256 >> log2_phases
+  int64_t blocks;
+};
+
+// Enough threads for the chip: the fewest phases that give kPairThreads, at most 32.
+constexpr int64_t kPairThreads = 131072;
+PairSplit pair_split(int64_t n) {
+  PairSplit s;
+  s.log2_phases = 0;
+  while (s.log2_phases < 5 && (n << s.log2_phases) < kPairThreads) ++s.log2_phases;
+  s.atoms = kBlock >> s.log2_phases;
+  s.blocks = ceil_div(n, s.atoms);
+  return s;
+}
+
+// Sums the phases' values of every atom of the block in phase order; the result is in phase 0's threads.
+__device__ __forceinline__ void sum_phases(const PairSplit& sp, double (&v)[4]) {
+  if (sp.log2_phases == 0) return;
+  __shared__ double part[4][kBlock];
+#pragma unroll
+  for (int c = 0; c < 4; ++c) part[c][threadIdx.x] = v[c];
+  __syncthreads();
+  if ((int)threadIdx.x >= sp.atoms) return;
+  for (int ph = 1; ph < (1 << sp.log2_phases); ++ph) {
+#pragma unroll
+    for (int c = 0; c < 4; ++c) v[c] += part[c][ph * sp.atoms + threadIdx.x];
+  }
+}
+
+// 1/x for normal positive x by Newton-Raphson from the hardware's FP64 reciprocal approximation (about 20 bits): two
+// quadratic steps, the second's residual exact in its FMA, leave under 1 ulp. x = 0 gives NaN through inf * 0.
+__device__ __forceinline__ double recip(double x) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  y = fma(fma(-x, y, 1.0), y, y);
+  return fma(fma(-x, y, 1.0), y, y);
+}
+
+// LJ forces and energy, FP64. At 1M atoms (78 list entries each) the gathers bound it: L1 serves one 32-byte record per
+// cycle, 0.29 ms for 82M entries, and the kernel takes 0.30 (one thread per atom over the caller's arrays, with branches
+// around each pair and three rounding instructions per minimum image: 0.67). Three gathers and the next list entries
+// in flight at 64 registers; more of either loses the occupancy that hides the FP64 chains (0.32 to 0.44 measured). An
+// 864-atom box: 52 -> 5.8 us; 256 atoms without a list: 92 -> 6.8. PACKED gathers one 256-bit record per neighbour, otherwise from the caller's arrays (the
+// entry point without a work buffer). ONE: a single species, its constants in registers; else the species-pair tables
+// are staged in shared memory (a kernel parameter indexed per thread serialises).
+template <bool DENSE, bool PACKED, bool ONE>
+__global__ void __launch_bounds__(kBlock, 4) k_lj64(const double* __restrict__ pos, const int32_t* __restrict__ sp,
+                                                  const Packed* __restrict__ pk, int64_t n, ImageBox box,
+                                                  const int32_t* __restrict__ nbr, const int32_t* __restrict__ nnb,
+                                                  int maxnb, const __grid_constant__ LJTab t, PairSplit split,
                                                   double* __restrict__ force, double* partials, unsigned int* ticket,
                                                   double* energy) {
-  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  double fx = 0.0, fy = 0.0, fz = 0.0, u = 0.0;
-  if (i < n) {
-    const double xi = pos[3 * i], yi = pos[3 * i + 1], zi = pos[3 * i + 2];
-    const int si = sp[i] * t.ns;
-    const int64_t m = DENSE ? n : (int64_t)min(nnb[i], maxnb);
-    for (int64_t k = 0; k < m; ++k) {
-      const int64_t j = DENSE ? k : (int64_t)nbr[nbr_slot(i, (int)k, maxnb)];
-      if (DENSE && j == i) continue;
-      double dx = sub(pos[3 * j], xi), dy = sub(pos[3 * j + 1], yi), dz = sub(pos[3 * j + 2], zi);
-      min_image3(dx, dy, dz, box);
-      const double r2 = norm2(dx, dy, dz);
-      const int p = si + sp[j];
-      const double e = t.eps[p];
-      if (r2 < t.rc2[p] && e > 0.0) {
-        const double ir2 = 1.0 / r2;
-        const double sr2 = t.sig2[p] * ir2;
-        const double sr6 = sr2 * sr2 * sr2;
-        u += 4.0 * e * (sr6 * sr6 - sr6 - t.shift6);
-        const double coef = -24.0 * e * (2.0 * sr6 * sr6 - sr6) * ir2;
-        fx += coef * dx;
-        fy += coef * dy;
-        fz += coef * dz;
-      }
+  __shared__ double tab[3][ONE ? 1 : ACS_MAX_SPECIES * ACS_MAX_SPECIES];
+  if (!ONE) {
+    for (int q = threadIdx.x; q < t.ns * t.ns; q += blockDim.x) {
+      tab[0][q] = t.eps[q];
+      tab[1][q] = t.sig2[q];
+      tab[2][q] = t.rc2[q];
     }
-    force[3 * i] = fx;
-    force[3 * i + 1] = fy;
-    force[3 * i + 2] = fz;
+    __syncthreads();
   }
-  double v[1] = {0.5 * u};
-  block_sum_finish<1>(v, partials, ticket, energy);
+  const int a = threadIdx.x & (split.atoms - 1), phase = threadIdx.x >> (8 - split.log2_phases);
+  const int phases = 1 << split.log2_phases;
+  const int64_t i = (int64_t)blockIdx.x * split.atoms + a;
+  constexpr int kU = 3;
+  double v[4] = {0.0, 0.0, 0.0, 0.0};
+  if (i < n) {
+    Packed me;
+    if (PACKED) {
+      me = ld_packed(pk + i);
+    } else {
+      me.x = pos[3 * i];
+      me.y = pos[3 * i + 1];
+      me.z = pos[3 * i + 2];
+    }
+    const int si = ONE ? 0 : (PACKED ? __double2loint(me.w) : sp[i]) * t.ns;
+    const double s1 = t.sig2[0], c1 = t.rc2[0];
+    // One block of U neighbours, without branches but for the boundary's minimum images: the terms of a neighbour
+    // outside the cutoff (3 in 10 list entries) are formed and dropped by a zero 1/r^2, so the U chains of dependent
+    // FP64 operations overlap; the energy shift is counted apart.
+    double cnt = 0.0;   // neighbours inside (ONE), or their sum of epsilon
+    auto block = [&](const Packed* o, const bool* ok, auto tag) {
+      constexpr int W = decltype(tag)::value;
+      double d[W][3];
+      bool near = true;
+#pragma unroll
+      for (int q = 0; q < W; ++q) {
+        d[q][0] = sub(o[q].x, me.x);
+        d[q][1] = sub(o[q].y, me.y);
+        d[q][2] = sub(o[q].z, me.z);
+        near = near && near_image(d[q][0], d[q][1], d[q][2], box);
+      }
+      if (!near) {
+#pragma unroll
+        for (int q = 0; q < W; ++q) image3(d[q][0], d[q][1], d[q][2], box);
+      }
+#pragma unroll
+      for (int q = 0; q < W; ++q) {
+        const double r2 = norm2(d[q][0], d[q][1], d[q][2]);
+        const int p = ONE ? 0 : si + __double2loint(o[q].w);
+        const double e = ONE ? 1.0 : tab[0][p];
+        const bool in = ok[q] && r2 < (ONE ? c1 : tab[2][p]) && e > 0.0;
+        const double ir2 = in ? recip(r2) : 0.0;
+        const double sr2 = (ONE ? s1 : tab[1][p]) * ir2;
+        const double sr6 = sr2 * sr2 * sr2;
+        const double w = fma(sr6, sr6, -sr6);
+        v[3] = ONE ? v[3] + w : fma(e, w, v[3]);
+        if (in) cnt += e;
+        const double c = (ONE ? ir2 : e * ir2) * fma(sr6, sr6, w);
+        if (in) {   // not 0 * d: an atom that is not finite has no neighbours and must not reach their sums
+          v[0] = fma(c, d[q][0], v[0]);
+          v[1] = fma(c, d[q][1], v[1]);
+          v[2] = fma(c, d[q][2], v[2]);
+        }
+      }
+    };
+    auto gather = [&](int32_t j) {
+      Packed o;
+      if (PACKED) {
+        o = ld_packed(pk + j);
+      } else {
+        o.x = pos[3 * (int64_t)j];
+        o.y = pos[3 * (int64_t)j + 1];
+        o.z = pos[3 * (int64_t)j + 2];
+        o.w = ONE ? 0.0 : __hiloint2double(0, sp[j]);
+      }
+      return o;
+    };
+    const int32_t* __restrict__ row = DENSE ? nullptr : nbr + nbr_slot(i, 0, maxnb);
+    const int64_t m = DENSE ? n : (int64_t)min(nnb[i], maxnb);
+    // list entry kq of this atom (-1 past the end); all atoms in turn without a list
+    auto entry = [&](int64_t kq) -> int32_t {
+      if (DENSE) return kq < m && kq != i ? (int32_t)kq : -1;
+      return kq < m ? __ldcs(row + kq * 32) : -1;
+    };
+    int32_t jn[kU];
+#pragma unroll
+    for (int q = 0; q < kU; ++q) jn[q] = entry(phase + q * phases);
+    for (int64_t k = phase; k < m; k += kU * phases) {
+      bool ok[kU];
+      Packed o[kU];
+#pragma unroll
+      for (int q = 0; q < kU; ++q) {   // a missing entry gathers the atom itself and is left out
+        ok[q] = jn[q] >= 0;
+        o[q] = gather(ok[q] ? jn[q] : (int32_t)i);
+      }
+#pragma unroll
+      for (int q = 0; q < kU; ++q) jn[q] = entry(k + (kU + q) * phases);   // the next block's entries
+      block(o, ok, std::integral_constant<int, kU>{});
+    }
+    const double e0 = ONE ? t.eps[0] : 1.0;
+    v[3] = 4.0 * e0 * (v[3] - t.shift6 * cnt);
+    v[0] *= -24.0 * e0;
+    v[1] *= -24.0 * e0;
+    v[2] *= -24.0 * e0;
+    if (ONE && !(e0 > 0.0)) v[0] = v[1] = v[2] = v[3] = 0.0;
+  }
+  sum_phases(split, v);
+  if (i < n && phase == 0) {
+    force[3 * i] = v[0];
+    force[3 * i + 1] = v[1];
+    force[3 * i + 2] = v[2];
+  }
+  double u[1] = {phase == 0 ? 0.5 * v[3] : 0.0};
+  block_sum_finish<1>(u, partials, ticket, energy);
+}
+
+template <bool PACKED, bool ONE>
+void launch_lj64(const double* pos, const int32_t* sp, const Packed* pk, int64_t n, const ImageBox& b, const int32_t* nbr,
+                 const int32_t* nnb, int maxnb, const LJTab& t, double* force, double* partials, unsigned int* ticket,
+                 double* energy, cudaStream_t s) {
+  const PairSplit split = pair_split(n);
+  if (nbr)
+    k_lj64<false, PACKED, ONE><<<(int)split.blocks, kBlock, 0, s>>>(pos, sp, pk, n, b, nbr, nnb, maxnb, t, split, force,
+                                                                    partials, ticket, energy);
+  else
+    k_lj64<true, PACKED, ONE><<<(int)split.blocks, kBlock, 0, s>>>(pos, sp, pk, n, b, nullptr, nullptr, 0, t, split,
+                                                                   force, partials, ticket, energy);
+}
+
+LJTab lj_tables(int n_species, const double* eps_tab, const double* sig_tab, double cutoff) {
+  LJTab t;
+  t.ns = n_species;
+  for (int a = 0; a < n_species * n_species; ++a) {
+    t.eps[a] = eps_tab[a];
+    t.sig2[a] = sig_tab[a] * sig_tab[a];                       // sig ** 2
+    const double rc = cutoff * sig_tab[a];
+    t.rc2[a] = rc * rc;                                        // (cutoff * sig) ** 2
+  }
+  const double c2 = cutoff * cutoff;
+  const double src6 = (1.0 / c2) * (1.0 / c2) * (1.0 / c2);
+  t.shift6 = src6 * src6 - src6;
+  return t;
 }
 
 template <bool DENSE>
@@ -906,7 +1093,24 @@ int acs_nlist_displacement(const double* pos, const double* pos0, int64_t n, con
   return launch_status();
 }
 
-size_t acs_force_work_bytes(int64_t n) { return align256(std::max<int64_t>(ceil_div(n, kBlock), 1) * 8) + 256; }
+// Energy partials (one per block of the pair kernels), ticket, packed positions; 256 bytes to align them in the
+// caller's buffer.
+static int64_t force_blocks(int64_t n) { return pair_split(std::max<int64_t>(n, 1)).blocks; }
+size_t acs_force_work_bytes(int64_t n) {
+  return align256(force_blocks(n) * 8) + 256 + align256((size_t)std::max<int64_t>(n, 1) * sizeof(Packed)) + 256;
+}
+
+// Carves a force call's work buffer and launches the packing kernel, which also clears the ticket.
+static int force_setup(const double* pos, const int32_t* sp, const double* q, int64_t n, void* work, size_t work_bytes,
+                       double** partials, unsigned int** ticket, Packed** pk, cudaStream_t s) {
+  if (work_bytes < acs_force_work_bytes(n) || !work) return ACS_ERR_WORKSPACE;
+  char* w = (char*)(((uintptr_t)work + 255) & ~(uintptr_t)255);
+  *partials = (double*)w; w += align256(force_blocks(n) * 8);
+  *ticket = (unsigned int*)w; w += 256;
+  *pk = (Packed*)w;
+  k_pack<<<(int)ceil_div(n, kBlock), kBlock, 0, s>>>(pos, sp, q, n, *pk, *ticket);
+  return launch_status();
+}
 
 static int reduce_setup(void* work, size_t work_bytes, size_t need, int64_t nblocks, int width, double** partials,
                         unsigned int** ticket, cudaStream_t s) {
@@ -924,28 +1128,17 @@ int acs_lj_fp64(const double* pos, const int32_t* sp, int64_t n, const double* b
       n_species > ACS_MAX_SPECIES || !(cutoff > 0.0) || (nbr && (!nnb || maxnb < 1)))
     return ACS_ERR_ARG;
   cudaStream_t s = (cudaStream_t)stream;
-  const int64_t nb = ceil_div(n, kBlock);
   double* partials;
   unsigned int* ticket;
-  int st = reduce_setup(work, work_bytes, acs_force_work_bytes(n), nb, 1, &partials, &ticket, s);
+  Packed* pk;
+  int st = force_setup(pos, sp, nullptr, n, work, work_bytes, &partials, &ticket, &pk, s);
   if (st) return st;
-  LJTab t;
-  t.ns = n_species;
-  for (int a = 0; a < n_species * n_species; ++a) {
-    t.eps[a] = eps_tab[a];
-    t.sig2[a] = sig_tab[a] * sig_tab[a];                       // sig ** 2
-    const double rc = cutoff * sig_tab[a];
-    t.rc2[a] = rc * rc;                                        // (cutoff * sig) ** 2
-  }
-  const double c2 = cutoff * cutoff;
-  const double src6 = (1.0 / c2) * (1.0 / c2) * (1.0 / c2);
-  t.shift6 = src6 * src6 - src6;
-  Box3 b = make_box(box3, periodic);
-  if (nbr)
-    k_lj64<false><<<(int)nb, kBlock, 0, s>>>(pos, sp, n, b, nbr, nnb, maxnb, t, force, partials, ticket, energy_dev);
+  const LJTab t = lj_tables(n_species, eps_tab, sig_tab, cutoff);
+  const ImageBox b = image_box(box3, periodic);
+  if (n_species == 1)
+    launch_lj64<true, true>(pos, sp, pk, n, b, nbr, nnb, maxnb, t, force, partials, ticket, energy_dev, s);
   else
-    k_lj64<true><<<(int)nb, kBlock, 0, s>>>(pos, sp, n, b, nullptr, nullptr, 0, t, force, partials, ticket,
-                                           energy_dev);
+    launch_lj64<true, false>(pos, sp, pk, n, b, nbr, nnb, maxnb, t, force, partials, ticket, energy_dev, s);
   return launch_status();
 }
 
@@ -1118,26 +1311,14 @@ extern "C" int acs_lj_fp64_noalloc(const double* pos, const int32_t* sp, int64_t
   int st = noalloc_scratch(&scratch);
   if (st) return st;
   cudaStream_t s = (cudaStream_t)stream;
-  const int64_t nb = ceil_div(n, kBlock);
   double* partials = (double*)scratch;
   unsigned int* ticket = (unsigned int*)((char*)scratch + kNoAllocMaxBlocks * 8);
   if (cudaMemsetAsync(ticket, 0, 4, s) != cudaSuccess) return ACS_ERR_CUDA;
-  LJTab t;
-  t.ns = n_species;
-  for (int a = 0; a < n_species * n_species; ++a) {
-    t.eps[a] = eps_tab[a];
-    t.sig2[a] = sig_tab[a] * sig_tab[a];
-    const double rc = cutoff * sig_tab[a];
-    t.rc2[a] = rc * rc;
-  }
-  const double c2 = cutoff * cutoff;
-  const double src6 = (1.0 / c2) * (1.0 / c2) * (1.0 / c2);
-  t.shift6 = src6 * src6 - src6;
-  Box3 b = make_box(box3, periodic);
-  if (nbr)
-    k_lj64<false><<<(int)nb, kBlock, 0, s>>>(pos, sp, n, b, nbr, nnb, maxnb, t, force, partials, ticket, energy_dev);
+  const LJTab t = lj_tables(n_species, eps_tab, sig_tab, cutoff);
+  const ImageBox b = image_box(box3, periodic);
+  if (n_species == 1)   // the same arithmetic as acs_lj_fp64, bit for bit
+    launch_lj64<false, true>(pos, sp, nullptr, n, b, nbr, nnb, maxnb, t, force, partials, ticket, energy_dev, s);
   else
-    k_lj64<true><<<(int)nb, kBlock, 0, s>>>(pos, sp, n, b, nullptr, nullptr, 0, t, force, partials, ticket,
-                                           energy_dev);
+    launch_lj64<false, false>(pos, sp, nullptr, n, b, nbr, nnb, maxnb, t, force, partials, ticket, energy_dev, s);
   return launch_status();
 }

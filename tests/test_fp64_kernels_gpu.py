@@ -8,6 +8,8 @@ import pytest
 
 pytestmark = pytest.mark.gpu
 
+EPS = 2.0 ** -53
+
 def _abi():
     import torch
 
@@ -113,3 +115,95 @@ def test_list_is_the_reference_filter_entry_by_entry(cells, n, periodic, kind, u
         s = status.cpu().numpy()
         assert s[0] == 1 and s[1] == maxnb and np.array_equal(nnb.cpu().numpy(), got_n)
         assert bool((nbr[(n + 31) // 32 * 32 * (maxnb - 1):] == -7).all())
+
+
+def _build_list(torch, L, st, p, g, maxnb):
+    n = len(p)
+    nbr = torch.empty((n + 31) // 32 * 32 * maxnb, dtype=torch.int32, device="cuda")
+    nnb = torch.empty(n, dtype=torch.int32, device="cuda")
+    status = torch.zeros(8, dtype=torch.int32, device="cuda")
+    work = torch.empty(L.acs_nlist_work_bytes(n, C.byref(g)), dtype=torch.uint8, device="cuda")
+    assert L.acs_nlist_build(p.data_ptr(), n, C.byref(g), maxnb, nbr.data_ptr(), nnb.data_ptr(), work.data_ptr(),
+                             work.numel(), status.data_ptr(), st) == 0
+    assert int(status[0].item()) == 0
+    return nbr, nnb
+
+
+def _pairs_within(pos, box, rc):
+    """(i, j, d_ij, r^2) of all ordered pairs with r < rc, in the reference's expression; row blocks."""
+    out = []
+    for a in range(0, len(pos), 400):
+        with np.errstate(invalid="ignore"):
+            d = pos[None, :, :] - pos[a:a + 400, None, :]
+            if box is not None:
+                d = d - box * np.round(d / box)
+            r2 = (d[..., 0] * d[..., 0] + d[..., 1] * d[..., 1]) + d[..., 2] * d[..., 2]
+            i, j = np.nonzero(r2 < rc ** 2)
+        keep = i + a != j
+        i, j = i[keep], j[keep]
+        out.append((i + a, j, d[i, j], r2[i, j]))
+    return [np.concatenate(x) for x in zip(*out)]
+
+
+def _scatter(n, i, x):
+    return np.stack([np.bincount(i, x[:, k], minlength=n) for k in range(3)], 1)
+
+
+# atoms: the pair kernels' splits change at 8, 4096 (32 -> 16 phases at 131,072 threads), 8192; blocks end ragged
+@pytest.mark.parametrize("n", [1, 2, 7, 9, 255, 257, 399, 4095, 4097, 8193])
+@pytest.mark.parametrize("species", [1, 3])
+@pytest.mark.parametrize("periodic", [True, False])
+@pytest.mark.parametrize("dense", [True, False])
+def test_lj_forces(n, species, periodic, dense):
+    """Forces and energy against NumPy over the same pairs: a term carries under 25 roundings of the same r^2, amplified
+    at most sevenfold by the powers, and an atom's sum under 200 additions, so an atom's force is within 400 eps of the
+    sum of its terms' magnitudes. One atom is not finite: it has no pairs."""
+    torch, L, st = _abi()
+    rng = np.random.default_rng(n + species)
+    box = np.array([1.0, 1.2, 0.9]) * (n / 0.8 / 1.08) ** (1 / 3)
+    if n > 20:   # a lattice with noise, some atoms left out
+        m = np.ceil((n / 1.08) ** (1 / 3) * np.array([1.0, 1.2, 0.9])).astype(int) + 1
+        grid = np.stack(np.meshgrid(*[np.arange(k) for k in m], indexing="ij"), -1).reshape(-1, 3)
+        pos = (grid[rng.permutation(len(grid))[:n]] + 0.5 + rng.normal(0, 0.06, (n, 3))) * box / m
+    else:
+        pos = rng.uniform(0, 1, (n, 3)) * box
+    if n > 8:
+        pos[5] = [np.nan, 0.1, 0.2] if periodic else [np.inf, 0.1, 0.2]
+    sp = rng.integers(0, species, n).astype(np.int32)
+    eps = np.array([[1.0, 0.8, 0.0], [0.8, 1.3, 0.7], [0.0, 0.7, 0.5]])[:species, :species].copy()
+    sig = np.array([[1.0, 0.95, 1.0], [0.95, 0.9, 0.85], [1.0, 0.85, 0.8]])[:species, :species].copy()
+    cutoff = 2.5
+    i, j, d, r2 = _pairs_within(pos, box if periodic else None, cutoff * sig.max())
+    e, s = eps[sp[i], sp[j]], sig[sp[i], sp[j]]
+    m = (r2 < (cutoff * s) ** 2) & (e > 0)
+    i, d, r2, e, s = i[m], d[m], r2[m], e[m], s[m]
+    s6 = (s ** 2 / r2) ** 3
+    c6 = cutoff ** -6.0
+    F = _scatter(n, i, (-24 * e * (2 * s6 ** 2 - s6) / r2)[:, None] * d)
+    mag = _scatter(n, i, (24 * e * (2 * s6 ** 2 + s6) / r2)[:, None] * np.abs(d))
+    U = 0.5 * np.sum(4 * e * (s6 ** 2 - s6 - (c6 ** 2 - c6)))
+    Umag = 0.5 * np.sum(4 * e * (s6 ** 2 + s6 + 1))
+    p, spd = torch.from_numpy(pos).cuda(), torch.from_numpy(sp).cuda()
+    nbr = nnb = None
+    maxnb = 0
+    if not dense:
+        if n < 2:
+            return
+        finite = pos[np.isfinite(pos).all(1)]
+        g = _grid(L, box if periodic else None, 2.8 * sig.max(), finite)
+        maxnb = 400
+        nbr, nnb = _build_list(torch, L, st, p, g, maxnb)
+    force = torch.full((n, 3), float("nan"), dtype=torch.float64, device="cuda")
+    energy = torch.full((1,), float("nan"), dtype=torch.float64, device="cuda")
+    work = torch.empty(L.acs_force_work_bytes(n) + 8, dtype=torch.uint8, device="cuda")
+    b = np.ascontiguousarray(box)
+    call = (p.data_ptr(), spd.data_ptr(), n, b.ctypes.data if periodic else None, int(periodic),
+            nbr.data_ptr() if nbr is not None else None, nnb.data_ptr() if nnb is not None else None, maxnb, species,
+            eps.ctypes.data, sig.ctypes.data, cutoff, force.data_ptr(), energy.data_ptr())
+    for extra in ((work.data_ptr() + 8, work.numel() - 8, st), (work.data_ptr() + 8, work.numel() - 8, st), (st,)):
+        fn = L.acs_lj_fp64 if len(extra) == 3 else L.acs_lj_fp64_noalloc
+        force.fill_(float("nan"))
+        assert fn(*call, *extra) == 0
+        got = force.cpu().numpy()
+        assert np.all(np.abs(got - F) <= 400 * EPS * mag)
+        assert abs(energy.item() - U) <= 400 * EPS * (Umag + 1e-300)
