@@ -18,6 +18,30 @@ def _abi():
     return torch, _lib.lib(), stream_handle()
 
 
+@pytest.mark.parametrize("n", [1, 31, 255, 256, 257, 65536, 65537, 300001])
+def test_conserved_sums(n):
+    """KE, P, L: every term passes through fewer than 64 roundings (products, shuffles, 8 warps, blocks / 256 strided
+    partials), so each sum is within 64 eps of the sum of its terms' magnitudes."""
+    torch, L, st = _abi()
+    rng = np.random.default_rng(n)
+    pos, vel = rng.uniform(0, 50, (n, 3)), rng.normal(0, 1, (n, 3))
+    sp = rng.integers(0, 2, n).astype(np.int32)
+    masses = np.array([1.5, 40.0])
+    p, v, s = (torch.from_numpy(x).cuda() for x in (pos, vel, sp))
+    out = torch.full((7,), float("nan"), dtype=torch.float64, device="cuda")
+    work = torch.empty(L.acs_reduce_work_bytes(n), dtype=torch.uint8, device="cuda")
+    for _ in range(2):   # the second call finds the ticket as the first left it
+        assert L.acs_reduce_conserved(p.data_ptr(), v.data_ptr(), s.data_ptr(), masses.ctypes.data, 2, n, out.data_ptr(),
+                                      work.data_ptr(), work.numel(), st) == 0
+    mom = masses[sp][:, None] * vel
+    ang = np.cross(pos, mom)
+    ref = np.concatenate([[0.5 * np.sum(mom * vel)], mom.sum(0), ang.sum(0)])
+    mag = np.concatenate([[0.5 * np.sum(np.abs(mom * vel))], np.abs(mom).sum(0),
+                          [np.sum(np.abs(pos[:, a] * mom[:, b]) + np.abs(pos[:, b] * mom[:, a]))
+                           for a, b in ((1, 2), (2, 0), (0, 1))]])
+    assert np.all(np.abs(out.cpu().numpy() - ref) <= 64 * EPS * mag + 64 * EPS * np.abs(ref))
+
+
 def _grid(L, box, rc, pos=None):
     from devinproj_b200 import _lib
     g = _lib.AcsGrid()
