@@ -231,3 +231,60 @@ def test_lj_forces(n, species, periodic, dense):
         got = force.cpu().numpy()
         assert np.all(np.abs(got - F) <= 400 * EPS * mag)
         assert abs(energy.item() - U) <= 400 * EPS * (Umag + 1e-300)
+
+
+# the splits as for LJ; exclusions, an atom that is not finite, uncharged atoms, alpha of zero
+@pytest.mark.parametrize("n", [1, 2, 9, 255, 399, 1024, 4097, 8193])
+@pytest.mark.parametrize("dense", [True, False])
+@pytest.mark.parametrize("alpha", [0.0, 0.8, 9.0])
+def test_dsf_forces(n, dense, alpha):
+    """Forces and energy against NumPy with SciPy's erfc over the same pairs. A pair's erfc and exponential carry the
+    rounding of alpha r, 2 (alpha r)^2 eps of their value, on top of a few eps each: within (60 + 4 (alpha rc)^2) eps of
+    the pair's term magnitudes, and an atom's sum adds under 200 roundings of the partial sums."""
+    from scipy.special import erfc
+    torch, L, st = _abi()
+    rng = np.random.default_rng(n)
+    rc, kc = 3.0, 1.7
+    box = np.array([1.1, 0.9, 1.0]) * max((n / 0.9) ** (1 / 3), 6.2)
+    m = np.ceil((n / 0.99) ** (1 / 3) * np.array([1.1, 0.9, 1.0])).astype(int) + 1
+    grid = np.stack(np.meshgrid(*[np.arange(k) for k in m], indexing="ij"), -1).reshape(-1, 3)
+    pos = (grid[rng.permutation(len(grid))[:n]] + 0.5 + rng.normal(0, 0.05, (n, 3))) * box / m
+    q = np.where(rng.random(n) < 0.5, 1.0, -1.2)
+    q[::7] = 0.0
+    if n > 8:
+        pos[5] = [np.nan, 0.1, 0.2]
+    i, j, d, r2 = _pairs_within(pos, box, rc)
+    ex = [] if n < 9 else [(0, int(k)) for k in set(j[i == 0][:3].tolist())] + [(1, n - 1)]
+    both = np.array(sorted({p for a, b in ex for p in ((a, b), (b, a))}), dtype=np.int64).reshape(-1, 2)
+    start = np.zeros(n + 1, np.int32)
+    start[1:] = np.cumsum(np.bincount(both[:, 0], minlength=n))
+    keep = ~np.isin(i * n + j, both[:, 0] * n + both[:, 1])
+    i, j, d, r = i[keep], j[keep], d[keep], np.sqrt(r2[keep])
+    c = 2 * alpha / np.sqrt(np.pi)
+    erc = erfc(alpha * rc)
+    sh = erc / rc ** 2 + c * np.exp(-(alpha * rc) ** 2) / rc
+    er, g = erfc(alpha * r), np.exp(-(alpha * r) ** 2)
+    qq = q[i] * q[j]
+    F = kc * _scatter(n, i, -(qq * ((er / r ** 2 + c * g / r) - sh) / r)[:, None] * d)
+    mag = kc * _scatter(n, i, (np.abs(qq) * ((er / r ** 2 + c * g / r) + sh) / r)[:, None] * np.abs(d))
+    self_c = erc / (2 * rc) + alpha / np.sqrt(np.pi)
+    U = kc * (0.5 * np.sum(qq * (er / r - erc / rc + sh * (r - rc))) - np.sum(q ** 2) * self_c)
+    Umag = kc * (0.5 * np.sum(np.abs(qq) * (er / r + erc / rc + sh * (rc - r))) + np.sum(q ** 2) * self_c)
+    p, qd, sd, xd = (torch.from_numpy(x).cuda() for x in (pos, q, start, both[:, 1].astype(np.int32)))
+    nbr = nnb = None
+    maxnb = 0
+    if not dense:
+        if n < 2:
+            return
+        maxnb = 400
+        nbr, nnb = _build_list(torch, L, st, p, _grid(L, box, rc + 0.2), maxnb)
+    force = torch.full((n, 3), float("nan"), dtype=torch.float64, device="cuda")
+    energy = torch.full((1,), float("nan"), dtype=torch.float64, device="cuda")
+    work = torch.empty(L.acs_force_work_bytes(n), dtype=torch.uint8, device="cuda")
+    assert L.acs_dsf_fp64(p.data_ptr(), qd.data_ptr(), n, np.ascontiguousarray(box).ctypes.data, 1,
+                          nbr.data_ptr() if nbr is not None else None, nnb.data_ptr() if nnb is not None else None, maxnb,
+                          sd.data_ptr() if ex else None, xd.data_ptr() if ex else None, alpha, rc, kc, force.data_ptr(),
+                          energy.data_ptr(), work.data_ptr(), work.numel(), st) == 0
+    tol = (260 + 4 * (alpha * rc) ** 2) * EPS
+    assert np.all(np.abs(force.cpu().numpy() - F) <= tol * mag + 1e-300)
+    assert abs(energy.item() - U) <= tol * Umag
