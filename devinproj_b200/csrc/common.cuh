@@ -1,6 +1,7 @@
 // Shared device helpers for the accusim_b200 kernels (sm_100a).
 #pragma once
 #include <cuda_runtime.h>
+#include <math.h>
 #include <stdint.h>
 #include <string.h>
 
@@ -65,7 +66,9 @@ struct Box3 {
 // quotient everywhere.
 struct ImageBox {
   double L[3], inv[3];
-  int near_hi[3];  // high word of 0.49 L: differences below it are their own minimum image
+  // high words of 0.49 L (differences below it are their own minimum image) and, for near_image1, of 0.49999 L, 0.50001 L
+  // and 1.49999 L (between the last two the image is one box away)
+  int near_hi[3], below_hi[3], above_hi[3], limit_hi[3];
   int periodic;
 };
 
@@ -74,10 +77,16 @@ inline ImageBox image_box(const double* edges3, int periodic) {
   for (int k = 0; k < 3; ++k) {
     b.L[k] = edges3 ? edges3[k] : 0.0;
     b.inv[k] = b.L[k] != 0.0 ? 1.0 / b.L[k] : 0.0;
-    const double near_d = b.L[k] > 0.0 && b.L[k] <= 1e300 ? 0.49 * b.L[k] : 0.0;
-    uint64_t bits;
-    memcpy(&bits, &near_d, 8);
-    b.near_hi[k] = (int)(bits >> 32);
+    const double L = b.L[k] > 0.0 && b.L[k] <= 1e300 ? b.L[k] : 0.0;
+    auto high = [](double x) {
+      uint64_t bits;
+      memcpy(&bits, &x, 8);
+      return (int)(bits >> 32);
+    };
+    b.near_hi[k] = high(0.49 * L);
+    b.below_hi[k] = high(0.49999 * L);
+    b.above_hi[k] = high(0.50001 * L) + 1;
+    b.limit_hi[k] = high(1.49999 * L);
   }
   b.periodic = periodic && edges3;
   return b;
@@ -123,6 +132,14 @@ __device__ __forceinline__ double recip_sqrt(double x) {
   return fma(fma(0.375, e, 0.5), y * e, y);
 }
 
+// The smallest double whose IEEE square root is at least r: r2 < square_reaching(r) decides as sqrt(r2) < r does.
+inline double square_reaching(double r) {
+  double t = r * r;
+  while (t > 0.0 && sqrt(t) >= r) t = nextafter(t, 0.0);
+  while (sqrt(t) < r) t = nextafter(t, HUGE_VAL);
+  return t;
+}
+
 // erfc(x) and exp(-x^2) for x >= 0. (1 + 2x) exp(x^2) erfc(x) is a smooth function of t = (x - k) / (x + k) over the
 // whole half line (Shepherd and Laframboise, Math. Comp. 36, 1981): with k = 3.75 its Chebyshev series, computed here
 // in extended precision to degree 23 and summed as two chains in t^2, is within 5.5e-17; the result is within 3 ulp of
@@ -161,6 +178,34 @@ __device__ __forceinline__ double erfc_exp(double x, double& gauss) {
   b = fma(b, t2, 8.22767384901452042e-02);
   b = fma(b, t2, -1.40240598585546966e-01);
   return fma(b, t, a) * (w * r) * gauss;
+}
+
+// An atom's position and one more value (species or charge) as one 32-byte sector, read by one 256-bit load: a pair
+// loop that gathers from the caller's arrays touches up to four sectors per neighbour in four loads.
+struct __align__(32) Packed {
+  double x, y, z, w;
+};
+
+__device__ __forceinline__ Packed ld_packed(const Packed* p) {
+  Packed v;
+  asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v.x), "=d"(v.y), "=d"(v.z), "=d"(v.w) : "l"(p));
+  return v;
+}
+
+// image3 for pairs that cross the box as often as not (all pairs of a periodic system): the choice between no shift and one
+// box by the high words, one addition per axis; anything else (within 1e-5 of half a box, unwrapped atoms) by image3. The
+// same results bit for bit.
+__device__ __forceinline__ void image3_any(double& dx, double& dy, double& dz, const ImageBox& b) {
+  const int hx = __double2hiint(dx) & 0x7fffffff, hy = __double2hiint(dy) & 0x7fffffff, hz = __double2hiint(dz) & 0x7fffffff;
+  const bool nx = hx < b.below_hi[0], ny = hy < b.below_hi[1], nz = hz < b.below_hi[2];
+  if ((nx || (hx >= b.above_hi[0] && hx < b.limit_hi[0])) && (ny || (hy >= b.above_hi[1] && hy < b.limit_hi[1])) &&
+      (nz || (hz >= b.above_hi[2] && hz < b.limit_hi[2]))) {
+    dx = sub(dx, nx ? 0.0 : copysign(b.L[0], dx));
+    dy = sub(dy, ny ? 0.0 : copysign(b.L[1], dy));
+    dz = sub(dz, nz ? 0.0 : copysign(b.L[2], dz));
+  } else {
+    image3(dx, dy, dz, b);
+  }
 }
 
 // Neighbour-list slot: warp-interleaved so that a warp of consecutive atoms reads 128 contiguous bytes.

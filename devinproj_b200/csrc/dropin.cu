@@ -557,18 +557,6 @@ struct DSFPar {
   double a, rc, rc2, k, c, erc, erc_rc, fshift, self_coef;
 };
 
-// An atom's position and one more value (species or charge) as one 32-byte sector, read by one 256-bit load: a pair
-// loop that gathers from the caller's arrays touches up to four sectors per neighbour in four loads.
-struct __align__(32) Packed {
-  double x, y, z, w;
-};
-
-__device__ __forceinline__ Packed ld_packed(const Packed* p) {
-  Packed v;
-  asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v.x), "=d"(v.y), "=d"(v.z), "=d"(v.w) : "l"(p));
-  return v;
-}
-
 // Packs positions with the species index (sp) or the charge (q) and clears the energy reduction's ticket.
 __global__ void k_pack(const double* __restrict__ pos, const int32_t* __restrict__ sp, const double* __restrict__ q,
                        int64_t n, Packed* __restrict__ out, unsigned int* ticket) {
@@ -1165,7 +1153,7 @@ int acs_dsf_fp64(const double* pos, const double* q, int64_t n, const double* bo
   DSFPar P;
   P.a = alpha;
   P.rc = rcut;
-  P.rc2 = rcut * rcut;
+  P.rc2 = square_reaching(rcut);
   P.k = k;
   P.c = 2.0 * alpha / sqrt(M_PI);
   P.erc = erfc(alpha * rcut);

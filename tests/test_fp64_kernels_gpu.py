@@ -13,9 +13,10 @@ EPS = 2.0 ** -53
 def _abi():
     import torch
 
-    from devinproj_b200 import _lib
+    from devinproj_b200 import ewald, learned
     from devinproj_b200.device import stream_handle
-    return torch, _lib.lib(), stream_handle()
+    ewald._bind()
+    return torch, learned._bind(), stream_handle()
 
 
 @pytest.mark.parametrize("n", [1, 31, 255, 256, 257, 65536, 65537, 300001])
@@ -288,3 +289,82 @@ def test_dsf_forces(n, dense, alpha):
     tol = (260 + 4 * (alpha * rc) ** 2) * EPS
     assert np.all(np.abs(force.cpu().numpy() - F) <= tol * mag + 1e-300)
     assert abs(energy.item() - U) <= tol * Umag
+
+
+def _ewald_vectors(kind, box, alpha):
+    kmax = {"wide": 17}.get(kind, 4)
+    m = np.arange(-kmax, kmax + 1)
+    N = np.stack(np.meshgrid(m, m, m, indexing="ij"), -1).reshape(-1, 3)
+    N = N[(np.sum(N ** 2, 1) <= kmax ** 2) & np.any(N != 0, 1)]
+    rng = np.random.default_rng(5)
+    if kind == "wide":          # integers beyond the tables
+        N = N[rng.permutation(len(N))[:301]]
+    if kind == "order":         # mirrored, but in no order, with unequal weights
+        N = N[rng.permutation(len(N))]
+    if kind == "half":          # no mirror images
+        N = N[(N[:, 0] > 0) | ((N[:, 0] == 0) & (N[:, 1] >= 0))]
+    if kind == "twice":         # a vector listed twice
+        N = np.concatenate([N, N[:3]])
+    if kind == "zero":          # the zero vector among them
+        N = np.concatenate([N, [[0, 0, 0]]])
+    kv = 2 * np.pi * N / box
+    if kind == "free":          # not reciprocal to the box
+        kv = kv * rng.uniform(0.9, 1.1, kv.shape)
+    k2 = np.maximum(np.sum(kv ** 2, 1), 1e-3)
+    w = np.exp(-k2 / (4 * alpha ** 2)) / k2
+    return np.ascontiguousarray(kv), w * (rng.uniform(0.5, 2, len(w)) if kind == "order" else 1.0)
+
+
+# atoms: below, at and above a tile of 32 and a block of 256; above the tiled kernel's range (few partners referenced)
+@pytest.mark.parametrize("n,kind", [(n, "lattice") for n in (1, 2, 31, 33, 255, 257, 700, 49153)]
+                         + [(300, k) for k in ("order", "half", "twice", "zero", "free", "wide")])
+def test_ewald_sum(n, kind):
+    """Forces, real-space energy and sum of w |S|^2 against NumPy. Real space as for DSF; a phase k.r carries 8 |k.r| eps
+    and a product of three factors a few eps, on S (of at most sum |q|) and on the force's factor."""
+    from scipy.special import erfc
+    torch, L, st = _abi()
+    rng = np.random.default_rng(n)
+    box = np.array([9.0, 11.0, 10.0])
+    pos = rng.uniform(-0.2, 1.2, (n, 3)) * box        # wrapped or not
+    q = rng.choice([-1.0, 1.0, 0.7], n)
+    rcut, alpha, kc = 4.4, 0.7, 1.3
+    kv, w = _ewald_vectors(kind, box, alpha)
+    rows = np.arange(n) if n < 1000 else np.r_[0:40, n - 40:n]
+    F, mag = np.zeros((len(rows), 3)), np.zeros((len(rows), 3))
+    real = rmag = 0.0
+    for a, i in enumerate(rows):
+        d = pos - pos[i]
+        d = d - box * np.round(d / box)
+        r = np.sqrt((d[:, 0] * d[:, 0] + d[:, 1] * d[:, 1]) + d[:, 2] * d[:, 2])
+        m = (r < rcut) & (np.arange(n) != i)
+        d, r, qq = d[m], r[m], q[i] * q[m]
+        e = erfc(alpha * r)
+        t = (e / r + 2 * alpha / np.sqrt(np.pi) * np.exp(-(alpha * r) ** 2)) / r ** 2
+        F[a] = -np.sum((qq * t)[:, None] * d, 0)
+        mag[a] = np.sum((np.abs(qq) * t)[:, None] * np.abs(d), 0)
+        real += 0.5 * np.sum(qq * e / r)
+        rmag += 0.5 * np.sum(np.abs(qq) * e / r)
+    ph = pos @ kv.T
+    S = (q[:, None] * np.exp(1j * ph)).sum(0)
+    rec = np.sum(w * np.abs(S) ** 2)
+    V = float(np.prod(box))
+    im = np.imag(np.conj(S)[None, :] * np.exp(1j * ph[rows]))
+    F += 4 * np.pi / V * q[rows][:, None] * ((w * im) @ kv)
+    wide = (8 * np.abs(ph).max() + 100) * EPS
+    Q = np.abs(q).sum()
+    tol = (300 + 4 * (alpha * rcut) ** 2) * EPS * mag + 2 * wide * 4 * np.pi / V * np.abs(q[rows])[:, None] * Q * (w @ np.abs(kv))
+    dev = [torch.from_numpy(np.ascontiguousarray(x)).cuda() for x in (pos, q, kv, w)]
+    force = torch.full((n, 3), float("nan"), dtype=torch.float64, device="cuda")
+    e3 = torch.full((3,), float("nan"), dtype=torch.float64, device="cuda")
+    nbytes = L.acs_ewald_work_bytes(n, len(w))
+    work = torch.empty(nbytes + 8, dtype=torch.uint8, device="cuda")
+    for _ in range(2):
+        assert L.acs_ewald_fp64(dev[0].data_ptr(), dev[1].data_ptr(), n, box.ctypes.data, dev[2].data_ptr(),
+                                dev[3].data_ptr(), len(w), alpha, rcut, kc, force.data_ptr(), e3.data_ptr(),
+                                work.data_ptr() + 8, nbytes, st) == 0
+        got = force.cpu().numpy()[rows] / kc
+        assert np.all(np.abs(got - F) <= tol)
+        e = e3.cpu().numpy()
+        if n < 1000:
+            assert abs(e[0] - real) <= (300 + 4 * (alpha * rcut) ** 2) * EPS * rmag
+        assert abs(e[1] - rec) <= 2 * wide * np.sum(w) * Q ** 2
