@@ -25,17 +25,6 @@ __device__ __forceinline__ double div(double a, double b) { return __ddiv_rn(a, 
 // d -= box * np.round(d / box)   (np.round: half to even == rint)
 __device__ __forceinline__ double min_image(double d, double box) { return sub(d, mul(box, rint(div(d, box)))); }
 
-// The same, bit for bit, with a multiply by 1/box in place of the division for almost every pair: t = d (1/box)
-// differs from the IEEE quotient d / box by under 3e-16 |d / box|, and rint only changes at half-integers, so
-// rint(t) is rint(d / box) unless t lies within 1e-9 of a half-integer (or |t| is huge); there the quotient
-// decides as in the reference.
-__device__ __forceinline__ double min_image(double d, double box, double inv_box) {
-  const double t = d * inv_box;
-  const double f = fabs(t - trunc(t));
-  const double k = (fabs(f - 0.5) > 1e-9 && fabs(t) < 1e6) ? rint(t) : rint(div(d, box));
-  return sub(d, mul(box, k));
-}
-
 // The same, bit for bit, without the division for almost every pair. A difference below 0.49 box (compared through
 // the high words, on the integer pipe) has k = 0 and stays as it is. Otherwise t = d (1/box) differs from the IEEE
 // quotient d / box by under 3e-16 |d / box|, and rint only changes at half-integers, so rint(t) is rint(d / box)
@@ -56,17 +45,11 @@ __device__ __forceinline__ double norm2(double dx, double dy, double dz) {
   return add(add(mul(dx, dx), mul(dy, dy)), mul(dz, dz));
 }
 
-struct Box3 {
-  double L[3];
-  double inv[3];   // 1 / L, for min_image's multiply
-  int periodic;
-};
-
 // A box with the constants the pair kernels' minimum image uses; an edge that is not a positive number takes the
 // quotient everywhere.
 struct ImageBox {
   double L[3], inv[3];
-  // high words of 0.49 L (differences below it are their own minimum image) and, for near_image1, of 0.49999 L, 0.50001 L
+  // high words of 0.49 L (differences below it are their own minimum image) and, for image3_any, of 0.49999 L, 0.50001 L
   // and 1.49999 L (between the last two the image is one box away)
   int near_hi[3], below_hi[3], above_hi[3], limit_hi[3];
   int periodic;
@@ -103,14 +86,6 @@ __device__ __forceinline__ void image3(double& dx, double& dy, double& dz, const
     dx = image1(dx, b.L[0], b.inv[0], b.near_hi[0]);
     dy = image1(dy, b.L[1], b.inv[1], b.near_hi[1]);
     dz = image1(dz, b.L[2], b.inv[2], b.near_hi[2]);
-  }
-}
-
-__device__ __forceinline__ void min_image3(double& dx, double& dy, double& dz, const Box3& b) {
-  if (b.periodic) {
-    dx = min_image(dx, b.L[0], b.inv[0]);
-    dy = min_image(dy, b.L[1], b.inv[1]);
-    dz = min_image(dz, b.L[2], b.inv[2]);
   }
 }
 

@@ -368,3 +368,43 @@ def test_ewald_sum(n, kind):
         if n < 1000:
             assert abs(e[0] - real) <= (300 + 4 * (alpha * rcut) ** 2) * EPS * rmag
         assert abs(e[1] - rec) <= 2 * wide * np.sum(w) * Q ** 2
+
+
+# boxes whose cells at rmax are one, three (the image found per pair) and four and more per axis; ragged counts
+@pytest.mark.parametrize("box,n", [((2.1, 2.3, 2.0), 65), ((3.1, 3.5, 3.3), 700), ((4.2, 6.1, 5.0), 2500), ((9.0, 4.1, 7.7), 5003),
+                                   ((2.5, 8.0, 3.9), 33)])
+@pytest.mark.parametrize("species", [-1, 1])
+@pytest.mark.parametrize("bins", [1, 100, 8192])
+def test_pair_histogram(box, n, species, bins):
+    """Counts against NumPy's histogram of the reference's distances; distances on bin edges and at rmax, atoms outside the
+    box. Exact."""
+    torch, L, st = _abi()
+    rng = np.random.default_rng(n)
+    box, rmax = np.array(box), 1.0
+    pos = rng.uniform(0, 1, (n, 3)) * box
+    pos[: n // 4] = np.round(pos[: n // 4] * 50) / 50          # distances on edges
+    pos[-9:] += rng.integers(-2, 3, (9, 3)) * box
+    sp = rng.integers(0, 2, n).astype(np.int32)
+    g = _grid(L, box, rmax)
+    # pairs the cell grid meets: an atom outside the box sits in an edge cell
+    t = pos / np.array(g.span) * np.array(g.ncell)
+    nc = np.array(g.ncell)
+    cell = np.where(t >= 1, np.where(t >= nc - 1, nc - 1, np.floor(t)), 0).astype(int)
+    r = []
+    for i in range(n - 1):
+        dc = cell[i + 1:] - cell[i]
+        dc = np.where(nc >= 3, (dc + 1) % nc - 1, dc)
+        m = np.all(np.abs(dc) <= 1, 1)
+        if species >= 0:
+            m &= (sp[i + 1:] == species) & (sp[i] == species)
+        d = pos[i + 1:][m] - pos[i]
+        d = d - box * np.round(d / box)
+        r.append(np.sqrt((d[:, 0] * d[:, 0] + d[:, 1] * d[:, 1]) + d[:, 2] * d[:, 2]))
+    r = np.concatenate(r)
+    ref = np.histogram(r[r <= rmax], bins=bins, range=(0, rmax))[0]
+    p, s = torch.from_numpy(pos).cuda(), torch.from_numpy(sp).cuda()
+    hist = torch.full((bins,), -1, dtype=torch.int64, device="cuda")
+    work = torch.empty(L.acs_rdf_work_bytes(n, C.byref(g)), dtype=torch.uint8, device="cuda")
+    assert L.acs_rdf_hist(p.data_ptr(), s.data_ptr(), n, C.byref(g), species, bins, rmax, hist.data_ptr(), work.data_ptr(),
+                          work.numel(), st) == 0
+    assert np.array_equal(hist.cpu().numpy(), ref)
