@@ -408,3 +408,43 @@ def test_pair_histogram(box, n, species, bins):
     assert L.acs_rdf_hist(p.data_ptr(), s.data_ptr(), n, C.byref(g), species, bins, rmax, hist.data_ptr(), work.data_ptr(),
                           work.numel(), st) == 0
     assert np.array_equal(hist.cpu().numpy(), ref)
+
+
+# neighbours: none, under a warp's 32, at and over the 128 staged at a time, both species, boxes of one and more cells
+@pytest.mark.parametrize("n,edge", [(1, 21.0), (2, 21.0), (9, 24.0), (130, 21.0), (300, 20.5), (1001, 33.0)])
+def test_descriptors(n, edge):
+    """Invariants and vector features against FP64. FP32 distances (2 ulp) enter the Gaussians with a slope of at most
+    0.6 / s and the approximate exponential and cosine are within 4e-7 and 1e-6, so a neighbour's term is off by under
+    1e-5 of the cutoff's size; X is rounded to BF16 on top."""
+    torch, L, st = _abi()
+    rng = np.random.default_rng(n)
+    box = np.array([1.0, 1.1, 0.95]) * edge
+    rc, r0 = 10.0, 1.8
+    dmu = (rc - r0) / 31
+    pos = rng.uniform(0, 1, (n, 3)) * box
+    if n == 2:
+        pos[1] = (pos[0] + [0.0, 0.0, 2.0]) % box
+    sp = rng.integers(0, 2, n).astype(np.int32)
+    i, j, d, r2 = _pairs_within(pos, box, rc)
+    r = np.sqrt(r2)
+    mu = r0 + dmu * np.arange(32)
+    g = np.exp(-(r[:, None] - mu) ** 2 / (2 * dmu ** 2)) * 0.5 * (np.cos(np.pi * r / rc) + 1)[:, None]
+    D, V, count = np.zeros((n, 2, 32)), np.zeros((n, 2, 32, 3)), np.zeros((n, 2, 1))
+    np.add.at(D, (i, sp[j]), g)
+    np.add.at(V, (i, sp[j]), g[:, :, None] * (d / r[:, None])[:, None, :])
+    np.add.at(count, (i, sp[j]), 1.0)
+    mean, inv = rng.normal(0, 1, 64).astype(np.float32), rng.uniform(0.5, 2, 64).astype(np.float32)
+    p, s = torch.from_numpy(pos).cuda(), torch.from_numpy(sp).cuda()
+    nbr, nnb = _build_list(torch, L, st, p, _grid(L, box, rc), 512)
+    par = np.array([r0, dmu, 1 / (2 * dmu ** 2), rc, 0, 0], np.float32)
+    X = torch.full((n, 80), float("nan"), dtype=torch.bfloat16, device="cuda")
+    W = torch.full((n, 64, 3), float("nan"), dtype=torch.float32, device="cuda")
+    md, vd = torch.from_numpy(mean).cuda(), torch.from_numpy(inv).cuda()
+    assert L.acs_descriptors(p.data_ptr(), s.data_ptr(), n, box.ctypes.data, 1, nbr.data_ptr(), nnb.data_ptr(), 512,
+                             par.ctypes.data, md.data_ptr(), vd.data_ptr(), X.data_ptr(), W.data_ptr(), st) == 0
+    x = X.float().cpu().numpy()
+    tol = 1e-5 * (count + 1)
+    assert np.all(np.abs(W.cpu().numpy().reshape(n, 2, 32, 3) - V) <= tol[..., None])
+    ref = (D.reshape(n, 64) - mean) * inv
+    assert np.all(np.abs(x[:, :64] - ref) <= 2.0 ** -8 * np.abs(ref) + 2 * np.repeat(tol, 32, 2).reshape(n, 64))
+    assert np.array_equal(x[:, 64:], np.eye(16, dtype=np.float32)[[15]].repeat(n, 0) + np.eye(16, dtype=np.float32)[sp])
