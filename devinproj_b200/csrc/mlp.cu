@@ -244,10 +244,6 @@ __device__ __forceinline__ float dsilu(float z) {
   return s * (1.0f + z * (1.0f - s));
 }
 
-__device__ __forceinline__ void put(unsigned char* sm, uint32_t base, int r, int k, int R, float v) {
-  *reinterpret_cast<bf16*>(sm + base + umma::tile_offset(r, k, R)) = __float2bfloat16(v);
-}
-
 // Row-major [R x K] BF16 (global, 16-byte aligned rows) -> canonical tile: each 8-element row segment of a core
 // matrix is 16 contiguous bytes, moved with one asynchronous 16-byte copy (all of a thread's copies are in
 // flight together; cp_async_wait() completes them). Rows >= rows_valid are zero-filled.
@@ -266,17 +262,6 @@ __device__ __forceinline__ void load_tile(unsigned char* sm, uint32_t base, cons
 __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.commit_group;" ::: "memory");
   asm volatile("cp.async.wait_all;" ::: "memory");
-}
-
-// One row of FP32 values (64) -> BF16 row r of a canonical tile, 16 bytes per store.
-__device__ __forceinline__ void put_row64(unsigned char* sm, uint32_t base, int r, int R, const float* v) {
-#pragma unroll
-  for (int k8 = 0; k8 < 8; ++k8) {
-    __nv_bfloat162 p[4];
-#pragma unroll
-    for (int q = 0; q < 4; ++q) p[q] = __floats2bfloat162_rn(v[8 * k8 + 2 * q], v[8 * k8 + 2 * q + 1]);
-    *reinterpret_cast<uint4*>(sm + base + umma::tile_offset(r, 8 * k8, R)) = *reinterpret_cast<uint4*>(p);
-  }
 }
 
 // Issue D(+)= A[128 x K] B[N x K]^T (one elected thread), K in 16-wide slices.
@@ -315,182 +300,6 @@ __device__ __forceinline__ void smem_to_mma() {  // generic-proxy smem writes ->
   umma::fence_after();
 }
 
-__device__ __forceinline__ void read_row(uint32_t tmem, uint32_t col, int ncols, float* out) {
-  const int warp = threadIdx.x >> 5;
-  for (int c0 = 0; c0 < ncols; c0 += 16) {
-    float v[16];
-    umma::tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + col + (uint32_t)c0, v);
-#pragma unroll
-    for (int q = 0; q < 16; ++q) out[c0 + q] = v[q];
-  }
-}
-
-template <bool TRAIN>
-__global__ void __launch_bounds__(128, 1) k_mlp(const bf16* __restrict__ X, const float* __restrict__ V,
-                                                 const float* __restrict__ Y, int64_t n, MlpWeights W, float out_scale,
-                                                 float loss_scale, float* __restrict__ Fout, float* __restrict__ gpart,
-                                                 float* __restrict__ loss_part, int* status) {
-  extern __shared__ __align__(1024) unsigned char sm[];
-  __shared__ uint64_t mbar;
-  __shared__ uint32_t tslot;
-  constexpr uint32_t kH1 = MlpSmem::H1, kH2 = MlpSmem::H2;
-  const int t = threadIdx.x, warp = t >> 5;
-  const int64_t row0 = (int64_t)blockIdx.x * kTile;
-  const int64_t gi = row0 + t;
-  const bool valid = gi < n;
-  const int rows = (int)(n - row0 < kTile ? n - row0 : kTile);
-
-  if (t == 0) umma::mbar_init(&mbar, 1);
-
-  // operands: weights and this tile's inputs (rows past n are zero)
-  load_tile(sm, MlpSmem::W1, W.W1, kH, kIn);
-  load_tile(sm, MlpSmem::W2, W.W2, kH, kH);
-  load_tile(sm, MlpSmem::W3, W.W3, kOut, kH);
-  if (TRAIN) {
-    load_tile(sm, MlpSmem::W2T, W.W2T, kH, kH);
-    load_tile(sm, MlpSmem::W3T, W.W3T, kH, kOut);
-  }
-  load_tile(sm, MlpSmem::X, X + row0 * kIn, kTile, kIn, rows);
-  if (TRAIN) {  // weight-gradient A operand: rows 64..127 stay zero
-    for (int idx = t; idx < kTile * kTile; idx += blockDim.x) put(sm, MlpSmem::GT, idx / kTile, idx % kTile, kTile, 0.f);
-  }
-  if (warp == 0) umma::tmem_alloc(&tslot, kTCols);
-  cp_async_wait();
-  smem_to_mma();
-  const uint32_t tm = tslot;
-  Sync S{&mbar, 0u, status, true};
-
-  float z[64], c[64];
-  // ---- layer 1
-  if (t == 0) gemm(sm, tm + kTZ1, MlpSmem::X, MlpSmem::W1, kH, kIn, kH);
-  S.wait();
-  read_row(tm, kTZ1, kH, z);
-  for (int q = 0; q < kH; ++q) z[q] = silu(z[q]);
-  put_row64(sm, kH1, t, kTile, z);
-  if (TRAIN)
-    for (int q = 0; q < kH; ++q) put(sm, MlpSmem::H1T, q, t, kGradCols, z[q]);
-  if (TRAIN) {
-    put(sm, MlpSmem::H1T, 64, t, kGradCols, 1.f);
-    for (int q = 65; q < kGradCols; ++q) put(sm, MlpSmem::H1T, q, t, kGradCols, 0.f);
-  }
-  smem_to_mma();
-  // ---- layer 2
-  if (t == 0) gemm(sm, tm + kTZ2, kH1, MlpSmem::W2, kH, kH, kH);
-  S.wait();
-  read_row(tm, kTZ2, kH, z);
-  for (int q = 0; q < kH; ++q) z[q] = silu(z[q] + W.b2[q]);
-  put_row64(sm, kH2, t, kTile, z);
-  if (TRAIN)
-    for (int q = 0; q < kH; ++q) put(sm, MlpSmem::H2T, q, t, kGradCols, z[q]);
-  if (TRAIN) {
-    put(sm, MlpSmem::H2T, 64, t, kGradCols, 1.f);
-    for (int q = 65; q < kGradCols; ++q) put(sm, MlpSmem::H2T, q, t, kGradCols, 0.f);
-  }
-  smem_to_mma();
-  // ---- layer 3: coefficients, contraction with the vector features
-  if (t == 0) gemm(sm, tm + kTC, kH2, MlpSmem::W3, kOut, kH, kOut);
-  S.wait();
-  read_row(tm, kTC, kOut, c);
-  float F[3] = {0.f, 0.f, 0.f};
-  if (valid) {
-    const float* vrow = V + gi * kOut * 3;
-    for (int q = 0; q < kOut; ++q) {
-      c[q] += W.b3[q];
-      F[0] += c[q] * vrow[3 * q];
-      F[1] += c[q] * vrow[3 * q + 1];
-      F[2] += c[q] * vrow[3 * q + 2];
-    }
-    if (Fout) {
-      Fout[3 * gi] = out_scale * F[0];
-      Fout[3 * gi + 1] = out_scale * F[1];
-      Fout[3 * gi + 2] = out_scale * F[2];
-    }
-  }
-  if (TRAIN) {
-    // loss = loss_scale * sum |F - Y|^2 over valid rows; dF = 2 loss_scale (F - Y)
-    float dF[3] = {0.f, 0.f, 0.f}, l = 0.f;
-    if (valid) {
-      for (int d = 0; d < 3; ++d) {
-        const float r = F[d] - Y[3 * gi + d];
-        l += r * r;
-        dF[d] = 2.0f * loss_scale * r;
-      }
-    }
-    for (int o = 16; o > 0; o >>= 1) l += __shfl_down_sync(0xffffffffu, l, o);
-    if ((t & 31) == 0) loss_part[blockIdx.x * 4 + warp] = loss_scale * l;
-    const float* vrow = V + (valid ? gi : 0) * kOut * 3;
-    for (int q = 0; q < kOut; ++q) {  // dC = dF . V_c
-      const float g = valid ? dF[0] * vrow[3 * q] + dF[1] * vrow[3 * q + 1] + dF[2] * vrow[3 * q + 2] : 0.f;
-      put(sm, MlpSmem::G, t, q, kTile, g);
-      put(sm, MlpSmem::GT, q, t, kTile, g);
-    }
-    smem_to_mma();
-    float* gp = gpart + (int64_t)blockIdx.x * (3 * kH * kGradCols);
-    // ---- dW3 (+ db3 in column 64), dH2
-    if (t == 0) {
-      gemm(sm, tm + kTdW, MlpSmem::GT, MlpSmem::H2T, kGradCols, kTile, kGradCols);
-      gemm(sm, tm + kTdH, MlpSmem::G, MlpSmem::W3T, kH, kOut, kH);
-    }
-    S.wait();
-    {
-      float w[kGradCols];
-      read_row(tm, kTdW, kGradCols, w);
-      if (t < kOut)
-        for (int q = 0; q < kGradCols; ++q) gp[2 * kH * kGradCols + t * kGradCols + q] = w[q];
-    }
-    read_row(tm, kTdH, kH, c);   // dH2
-    read_row(tm, kTZ2, kH, z);   // Z2 without b2
-    umma::fence_before();
-    __syncthreads();
-    for (int q = 0; q < kH; ++q) {
-      const float g = c[q] * dsilu(z[q] + W.b2[q]);
-      put(sm, MlpSmem::G, t, q, kTile, g);
-      put(sm, MlpSmem::GT, q, t, kTile, g);
-    }
-    smem_to_mma();
-    // ---- dW2 (+ db2), dH1
-    if (t == 0) {
-      gemm(sm, tm + kTdW, MlpSmem::GT, MlpSmem::H1T, kGradCols, kTile, kGradCols);
-      gemm(sm, tm + kTdH, MlpSmem::G, MlpSmem::W2T, kH, kH, kH);
-    }
-    S.wait();
-    {
-      float w[kGradCols];
-      read_row(tm, kTdW, kGradCols, w);
-      if (t < kH)
-        for (int q = 0; q < kGradCols; ++q) gp[1 * kH * kGradCols + t * kGradCols + q] = w[q];
-    }
-    read_row(tm, kTdH, kH, c);   // dH1
-    read_row(tm, kTZ1, kH, z);   // Z1
-    umma::fence_before();
-    __syncthreads();
-    for (int q = 0; q < kH; ++q) put(sm, MlpSmem::GT, q, t, kTile, c[q] * dsilu(z[q]));
-    for (int k = 0; k < kIn; ++k) {  // X^T into the (now free) H2T buffer
-      const bf16 v = *reinterpret_cast<const bf16*>(sm + MlpSmem::X + umma::tile_offset(t, k, kTile));
-      *reinterpret_cast<bf16*>(sm + MlpSmem::H2T + umma::tile_offset(k, t, kGradCols)) = v;
-    }
-    smem_to_mma();
-    // ---- dW1 (bias = column 79)
-    if (t == 0) gemm(sm, tm + kTdW, MlpSmem::GT, MlpSmem::H2T, kGradCols, kTile, kGradCols);
-    S.wait();
-    {
-      float w[kGradCols];
-      read_row(tm, kTdW, kGradCols, w);
-      if (t < kH)
-        for (int q = 0; q < kGradCols; ++q) gp[t * kGradCols + q] = w[q];
-    }
-  }
-  umma::fence_before();
-  __syncthreads();
-  if (warp == 0) umma::tmem_free(tm, kTCols);
-}
-
-// Inference on one 128-ion tile with 256 threads. Warps w and w + 4 share TMEM lane quadrant w % 4 (rows
-// 32 (w % 4) + lane) and split every epilogue's columns: half h = w / 4 takes [32 h, 32 h + 32). The tile's
-// vector features stream into shared memory (bulk copies) behind the three layers; the two halves of the
-// contraction F = sum_c C_c V_c meet in shared memory.
-constexpr uint32_t kInfCols = 256;  // TMEM: Z1 [0, 64), Z2 [64, 128), C [128, 192)
-
 __device__ __forceinline__ void read32(uint32_t tmem, int quad, uint32_t col, float* out) {
   float v[16];
   umma::tmem_ld16(tmem + ((uint32_t)(quad * 32) << 16) + col, v);
@@ -511,6 +320,234 @@ __device__ __forceinline__ void put_row32(unsigned char* sm, uint32_t base, int 
     *reinterpret_cast<uint4*>(sm + base + umma::tile_offset(r, 8 * (k8_0 + k8), R)) = *reinterpret_cast<uint4*>(p);
   }
 }
+
+// Transposed copy of columns [c0, c0 + 8 blocks) of this warp's rows [r0, r0 + 32) from one canonical tile (rs rows) to
+// another (rd rows): 8x8 BF16 blocks, read transposed and written four at a time.
+__device__ __forceinline__ void transpose(unsigned char* sm, uint32_t src, int rs, uint32_t dst, int rd, int r0, int c0,
+                                          int blocks) {
+  const int lane = threadIdx.x & 31, row = r0 + lane, r8 = r0 + (lane & 24), q = lane & 7;
+  __syncwarp();
+  for (int b = 0; b < blocks; ++b) {
+    const int c = c0 + 8 * b;
+    const uint32_t from = umma::smem_u32(sm + src + umma::tile_offset(row, c, rs));
+    const uint32_t to = umma::smem_u32(sm + dst + umma::tile_offset(c + q, r8, rd));
+    uint32_t m0, m1, m2, m3;
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(m0), "=r"(m1), "=r"(m2), "=r"(m3) : "r"(from) : "memory");
+    asm volatile("stmatrix.sync.aligned.m8n8.x4.shared.b16 [%0], {%1, %2, %3, %4};" ::"r"(to), "r"(m0), "r"(m1), "r"(m2),
+                 "r"(m3) : "memory");
+  }
+}
+
+// Rows [r0, r1) of a canonical tile of R rows and 128 columns set to one BF16 value.
+__device__ __forceinline__ void fill_rows(unsigned char* sm, uint32_t base, int r0, int r1, int R, float v) {
+  const __nv_bfloat162 two = __floats2bfloat162_rn(v, v);
+  const uint32_t w = *reinterpret_cast<const uint32_t*>(&two);
+  for (int t = threadIdx.x; t < (r1 - r0) * 16; t += blockDim.x)
+    *reinterpret_cast<uint4*>(sm + base + umma::tile_offset(r0 + t % (r1 - r0), 8 * (t / (r1 - r0)), R)) =
+        make_uint4(w, w, w, w);
+}
+
+// Forward, backward and the tile's weight gradients, 256 threads per tile of 128 ions, split as k_mlp_infer's: warps w and
+// w + 4 take the two halves of the columns of rows 32 (w % 4) + lane. A thread's half row of vector features (24 16-byte
+// loads issued at the start) stays in registers for the contraction and for its gradient; the row's contraction runs
+// through half 0, then half 1, so that its chain of additions is one. The transposed operands of the weight-gradient
+// MMAs are 8x8 block transposes of the row-major ones. With 128 threads, 4-byte loads of V twice over and an element
+// at a time of every transpose, 64 tiles took 60 us; 19 us so, mostly the latency of the six dependent MMA stages.
+__global__ void __launch_bounds__(256, 1) k_mlp_train(const bf16* __restrict__ X, const float* __restrict__ V,
+                                                      const float* __restrict__ Y, int64_t n, MlpWeights W,
+                                                      float loss_scale, float* __restrict__ gpart,
+                                                      float* __restrict__ loss_part, int* status, int wide) {
+  extern __shared__ __align__(1024) unsigned char sm[];
+  __shared__ uint64_t mbar;
+  __shared__ uint32_t tslot;
+  __shared__ float bias[128];          // b2, b3
+  __shared__ float contraction[3][kTile];
+  const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+  const int quad = warp & 3, half = warp >> 2;
+  const int row = 32 * quad + lane, r0 = 32 * quad, c0 = 32 * half;
+  const int64_t row0 = (int64_t)blockIdx.x * kTile;
+  const int64_t gi = row0 + row;
+  const bool valid = gi < n;
+  const int rows = (int)(n - row0 < kTile ? n - row0 : kTile);
+
+  if (t == 0) umma::mbar_init(&mbar, 1);
+  // this half's channels q in [32 h, 32 h + 32) are the row's FP32 elements [96 h, 96 h + 96)
+  float v[96];
+  {
+    const float* src = V + (valid ? gi : row0) * kOut * 3 + 96 * half;
+    if (wide) {
+#pragma unroll
+      for (int m = 0; m < 24; ++m) {
+        const float4 f = __ldg(reinterpret_cast<const float4*>(src) + m);
+        v[4 * m] = f.x;
+        v[4 * m + 1] = f.y;
+        v[4 * m + 2] = f.z;
+        v[4 * m + 3] = f.w;
+      }
+    } else {
+#pragma unroll
+      for (int m = 0; m < 96; ++m) v[m] = __ldg(src + m);
+    }
+  }
+  // operands: weights and this tile's inputs (rows past n are zero)
+  load_tile(sm, MlpSmem::W1, W.W1, kH, kIn);
+  load_tile(sm, MlpSmem::W2, W.W2, kH, kH);
+  load_tile(sm, MlpSmem::W3, W.W3, kOut, kH);
+  load_tile(sm, MlpSmem::W2T, W.W2T, kH, kH);
+  load_tile(sm, MlpSmem::W3T, W.W3T, kH, kOut);
+  load_tile(sm, MlpSmem::X, X + row0 * kIn, kTile, kIn, rows);
+  if (t < 128) bias[t] = t < 64 ? W.b2[t] : W.b3[t - 64];
+  fill_rows(sm, MlpSmem::GT, kH, kTile, kTile, 0.f);         // weight-gradient A operand: rows 64..127 stay zero
+  fill_rows(sm, MlpSmem::H1T, kH, kH + 1, kGradCols, 1.f);   // bias gradients: a row of ones, the rest zero
+  fill_rows(sm, MlpSmem::H1T, kH + 1, kGradCols, kGradCols, 0.f);
+  fill_rows(sm, MlpSmem::H2T, kH, kH + 1, kGradCols, 1.f);
+  fill_rows(sm, MlpSmem::H2T, kH + 1, kGradCols, kGradCols, 0.f);
+  if (warp == 0) umma::tmem_alloc(&tslot, kTCols);
+  cp_async_wait();
+  smem_to_mma();
+  const uint32_t tm = tslot;
+  Sync S{&mbar, 0u, status, true};
+  float z[32], c[32];
+  // ---- layer 1
+  if (t == 0) gemm(sm, tm + kTZ1, MlpSmem::X, MlpSmem::W1, kH, kIn, kH);
+  S.wait();
+  read32(tm, quad, kTZ1 + c0, z);
+#pragma unroll
+  for (int q = 0; q < 32; ++q) z[q] = silu(z[q]);
+  put_row32(sm, MlpSmem::H1, row, kTile, 4 * half, z);
+  transpose(sm, MlpSmem::H1, kTile, MlpSmem::H1T, kGradCols, r0, c0, 4);
+  smem_to_mma();
+  // ---- layer 2
+  if (t == 0) gemm(sm, tm + kTZ2, MlpSmem::H1, MlpSmem::W2, kH, kH, kH);
+  S.wait();
+  read32(tm, quad, kTZ2 + c0, z);
+#pragma unroll
+  for (int q = 0; q < 32; ++q) z[q] = silu(z[q] + bias[c0 + q]);
+  put_row32(sm, MlpSmem::H2, row, kTile, 4 * half, z);
+  transpose(sm, MlpSmem::H2, kTile, MlpSmem::H2T, kGradCols, r0, c0, 4);
+  smem_to_mma();
+  // ---- layer 3: coefficients, contraction with the vector features
+  if (t == 0) gemm(sm, tm + kTC, MlpSmem::H2, MlpSmem::W3, kOut, kH, kOut);
+  S.wait();
+  read32(tm, quad, kTC + c0, c);
+  auto contract = [&](float (&F)[3]) {
+#pragma unroll
+    for (int q = 0; q < 32; ++q) {
+      c[q] += bias[64 + c0 + q];
+      F[0] += c[q] * v[3 * q];
+      F[1] += c[q] * v[3 * q + 1];
+      F[2] += c[q] * v[3 * q + 2];
+    }
+  };
+  float F[3] = {0.f, 0.f, 0.f};
+  if (half == 0) {
+    contract(F);
+#pragma unroll
+    for (int d = 0; d < 3; ++d) contraction[d][row] = F[d];
+  }
+  __syncthreads();
+  // loss = loss_scale * sum |F - Y|^2 over valid rows; dF = 2 loss_scale (F - Y)
+  float dF[3] = {0.f, 0.f, 0.f};
+  if (half == 1) {
+#pragma unroll
+    for (int d = 0; d < 3; ++d) F[d] = contraction[d][row];
+    contract(F);
+    float l = 0.f;
+    if (valid) {
+#pragma unroll
+      for (int d = 0; d < 3; ++d) {
+        const float r = F[d] - Y[3 * gi + d];
+        l += r * r;
+        dF[d] = 2.0f * loss_scale * r;
+      }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) l += __shfl_down_sync(0xffffffffu, l, o);
+    if (lane == 0) loss_part[blockIdx.x * 4 + quad] = loss_scale * l;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) contraction[d][row] = dF[d];
+  }
+  __syncthreads();
+  if (half == 0) {
+#pragma unroll
+    for (int d = 0; d < 3; ++d) dF[d] = contraction[d][row];
+  }
+#pragma unroll
+  for (int q = 0; q < 32; ++q)   // dC = dF . V_c
+    c[q] = valid ? dF[0] * v[3 * q] + dF[1] * v[3 * q + 1] + dF[2] * v[3 * q + 2] : 0.f;
+  put_row32(sm, MlpSmem::G, row, kTile, 4 * half, c);
+  transpose(sm, MlpSmem::G, kTile, MlpSmem::GT, kTile, r0, c0, 4);
+  smem_to_mma();
+  float* gp = gpart + (int64_t)blockIdx.x * (3 * kH * kGradCols);
+  // one weight gradient (rows 0..63 of the accumulator, 80 columns, this half's 40) to its place
+  auto store_grad = [&](int layer) {
+    if (quad >= 2) return;
+    float w[40];
+#pragma unroll
+    for (int m = 0; m < 5; ++m) {
+      float x[8];
+      umma::tmem_ld8(tm + ((uint32_t)r0 << 16) + kTdW + 40u * half + 8u * m, x);
+#pragma unroll
+      for (int q = 0; q < 8; ++q) w[8 * m + q] = x[q];
+    }
+    float* dst = gp + (layer * kH + row) * kGradCols + 40 * half;
+    if (wide) {
+#pragma unroll
+      for (int m = 0; m < 10; ++m)
+        reinterpret_cast<float4*>(dst)[m] = make_float4(w[4 * m], w[4 * m + 1], w[4 * m + 2], w[4 * m + 3]);
+    } else {
+#pragma unroll
+      for (int m = 0; m < 40; ++m) dst[m] = w[m];
+    }
+  };
+  // ---- dW3 (+ db3 in column 64), dH2
+  if (t == 0) {
+    gemm(sm, tm + kTdW, MlpSmem::GT, MlpSmem::H2T, kGradCols, kTile, kGradCols);
+    gemm(sm, tm + kTdH, MlpSmem::G, MlpSmem::W3T, kH, kOut, kH);
+  }
+  S.wait();
+  read32(tm, quad, kTdH + c0, c);   // dH2
+  read32(tm, quad, kTZ2 + c0, z);   // Z2 without b2
+  store_grad(2);
+  umma::fence_before();
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < 32; ++q) c[q] = c[q] * dsilu(z[q] + bias[c0 + q]);
+  put_row32(sm, MlpSmem::G, row, kTile, 4 * half, c);
+  transpose(sm, MlpSmem::G, kTile, MlpSmem::GT, kTile, r0, c0, 4);
+  smem_to_mma();
+  // ---- dW2 (+ db2), dH1
+  if (t == 0) {
+    gemm(sm, tm + kTdW, MlpSmem::GT, MlpSmem::H1T, kGradCols, kTile, kGradCols);
+    gemm(sm, tm + kTdH, MlpSmem::G, MlpSmem::W2T, kH, kH, kH);
+  }
+  transpose(sm, MlpSmem::X, kTile, MlpSmem::H2T, kGradCols, r0, 40 * half, 5);   // X^T into the now free H2T buffer
+  S.wait();
+  read32(tm, quad, kTdH + c0, c);   // dH1
+  read32(tm, quad, kTZ1 + c0, z);   // Z1
+  store_grad(1);
+  umma::fence_before();
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < 32; ++q) c[q] = c[q] * dsilu(z[q]);
+  put_row32(sm, MlpSmem::G, row, kTile, 4 * half, c);
+  transpose(sm, MlpSmem::G, kTile, MlpSmem::GT, kTile, r0, c0, 4);
+  smem_to_mma();
+  // ---- dW1 (bias = column 79)
+  if (t == 0) gemm(sm, tm + kTdW, MlpSmem::GT, MlpSmem::H2T, kGradCols, kTile, kGradCols);
+  S.wait();
+  store_grad(0);
+  umma::fence_before();
+  __syncthreads();
+  if (warp == 0) umma::tmem_free(tm, kTCols);
+}
+
+// Inference on one 128-ion tile with 256 threads. Warps w and w + 4 share TMEM lane quadrant w % 4 (rows
+// 32 (w % 4) + lane) and split every epilogue's columns: half h = w / 4 takes [32 h, 32 h + 32). The tile's
+// vector features stream into shared memory (bulk copies) behind the three layers; the two halves of the
+// contraction F = sum_c C_c V_c meet in shared memory.
+constexpr uint32_t kInfCols = 256;  // TMEM: Z1 [0, 64), Z2 [64, 128), C [128, 192)
 
 __global__ void __launch_bounds__(256, 1) k_mlp_infer(const bf16* __restrict__ X, const float* __restrict__ V, int64_t n,
                                                       MlpWeights W, float out_scale, float* __restrict__ Fout,
@@ -606,7 +643,7 @@ __global__ void __launch_bounds__(256, 1) k_mlp_infer(const bf16* __restrict__ X
   if (warp == 0) umma::tmem_free(tm, kInfCols);
 }
 
-// Sum the per-tile gradient partials in tile order (deterministic) and take an Adam step on the FP32
+// Sum the per-tile gradient partials in tile order (deterministic; blocks of 64 threads reach all SMs) and take an Adam step on the FP32
 // master parameters; refresh the BF16 operand copies (W and the transposes of W2, W3).
 // Parameter vector: [W1 64x80 | W2aug 64x80 (cols 0..63 weights, 64 bias) | W3aug 64x80], FP32.
 __global__ void k_adam(const float* __restrict__ gpart, int ntiles, float* __restrict__ theta,
@@ -620,6 +657,7 @@ __global__ void k_adam(const float* __restrict__ gpart, int ntiles, float* __res
   const int layer = p / (kH * kGradCols), o = (p / kGradCols) % kH, col = p % kGradCols;
   const bool used = (layer == 0) ? true : (col <= 64);
   float g = 0.f;
+#pragma unroll 8
   for (int tl = 0; tl < ntiles; ++tl) g += gpart[(int64_t)tl * P + p];
   if (grad_out) grad_out[p] = g;
   if (!used) return;
@@ -707,25 +745,25 @@ int acs_mlp_train_step(const void* X, const float* V, const float* Y, int64_t n,
   if (gpart_bytes < acs_mlp_grad_bytes(n)) return ACS_ERR_WORKSPACE;
   cudaStream_t s = (cudaStream_t)stream;
   const size_t smem = MlpSmem::END;
-  if (cudaFuncSetAttribute(k_mlp<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+  if (cudaFuncSetAttribute(k_mlp_train, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
     return ACS_ERR_CUDA;
   const int ntiles = (int)ceil_div(n, kTile);
   MlpWeights W{(const bf16*)w5[0], (const bf16*)w5[1], (const bf16*)w5[2], (const bf16*)w5[3], (const bf16*)w5[4], b2, b3};
   const float loss_scale = 1.0f / (3.0f * (float)n);
-  k_mlp<true><<<ntiles, 128, smem, s>>>((const bf16*)X, V, Y, n, W, 1.0f, loss_scale, nullptr, gpart, loss_part,
-                                        status_dev);
+  const int wide = (((uintptr_t)V | (uintptr_t)gpart) & 15) == 0;   // 16-byte accesses to both
+  k_mlp_train<<<ntiles, 256, smem, s>>>((const bf16*)X, V, Y, n, W, loss_scale, gpart, loss_part, status_dev, wide);
   int st = launch_status();
   if (st) return st;
   if (lr > 0.f) {
     const float b1 = 0.9f, b2c = 0.999f;
     const float bc1 = 1.f - powf(b1, (float)step), bc2 = 1.f - powf(b2c, (float)step);
     const int P = 3 * kH * kGradCols;
-    k_adam<<<(P + 255) / 256, 256, 0, s>>>(gpart, ntiles, theta, adam_m, adam_v, lr, b1, b2c, 1e-8f, bc1, bc2,
+    k_adam<<<(P + 63) / 64, 64, 0, s>>>(gpart, ntiles, theta, adam_m, adam_v, lr, b1, b2c, 1e-8f, bc1, bc2,
                                            weight_decay, (bf16*)w5[0], (bf16*)w5[1], (bf16*)w5[2], (bf16*)w5[3],
                                            (bf16*)w5[4], b2, b3, grad_out);
   } else {
     const int P = 3 * kH * kGradCols;
-    k_adam<<<(P + 255) / 256, 256, 0, s>>>(gpart, ntiles, theta, adam_m, adam_v, 0.f, 0.9f, 0.999f, 1e-8f, 1.f, 1.f,
+    k_adam<<<(P + 63) / 64, 64, 0, s>>>(gpart, ntiles, theta, adam_m, adam_v, 0.f, 0.9f, 0.999f, 1e-8f, 1.f, 1.f,
                                            0.f, (bf16*)w5[0], (bf16*)w5[1], (bf16*)w5[2], (bf16*)w5[3], (bf16*)w5[4],
                                            b2, b3, grad_out);
   }

@@ -448,3 +448,53 @@ def test_descriptors(n, edge):
     ref = (D.reshape(n, 64) - mean) * inv
     assert np.all(np.abs(x[:, :64] - ref) <= 2.0 ** -8 * np.abs(ref) + 2 * np.repeat(tol, 32, 2).reshape(n, 64))
     assert np.array_equal(x[:, 64:], np.eye(16, dtype=np.float32)[[15]].repeat(n, 0) + np.eye(16, dtype=np.float32)[sp])
+
+
+# one row, a tile's last row, a full tile, one row into the next, many tiles
+@pytest.mark.parametrize("n", [1, 127, 128, 129, 1000])
+def test_training_step_gradient(n):
+    """Loss and gradient against FP64 of the same BF16 weights and inputs (activations and their gradients are rounded to
+    BF16, 2^-9 each through three layers: 3e-2 of the gradient's norm, 1e-2 of the loss); buffers that are not
+    16-byte aligned give the same bits."""
+    torch, L, st = _abi()
+    rng = np.random.default_rng(n)
+    th = rng.normal(0, 0.12, (3, 64, 80)).astype(np.float32)
+    th[1:, :, 65:] = 0
+    X = rng.normal(0, 1, (n, 80))
+    X[:, 66:79], X[:, 79] = 0, 1
+    V, Y = rng.normal(0, 0.7, (n, 64, 3)).astype(np.float32), rng.normal(0, 0.5, (n, 3)).astype(np.float32)
+    Xb = torch.from_numpy(X).to(torch.bfloat16)
+    q = torch.from_numpy(th).double()
+    q[0] = torch.from_numpy(th[0]).to(torch.bfloat16).double()
+    q[1:, :, :64] = torch.from_numpy(th[1:, :, :64]).to(torch.bfloat16).double()
+    q.requires_grad_(True)
+    silu = torch.nn.functional.silu
+    h = silu(silu(Xb.double() @ q[0].T) @ q[1][:, :64].T + q[1][:, 64])
+    F = torch.einsum("nc,ncd->nd", h @ q[2][:, :64].T + q[2][:, 64], torch.from_numpy(V).double())
+    loss = ((F - torch.from_numpy(Y).double()) ** 2).sum() / (3 * n)
+    loss.backward()
+    ref = q.grad.numpy().reshape(-1)
+    out = []
+    for shift in (0, 4):
+        def device(a):
+            b = torch.empty(a.nbytes + 16, dtype=torch.uint8, device="cuda")
+            t = b[shift:shift + a.nbytes].view(torch.float32).view(a.shape)
+            return t.copy_(torch.from_numpy(a))
+        w = torch.from_numpy(th).cuda()
+        ws = [x.contiguous().to(torch.bfloat16) for x in (w[0], w[1][:, :64], w[2][:, :64], w[1][:, :64].T, w[2][:, :64].T)]
+        w5 = (C.c_void_p * 5)(*[x.data_ptr() for x in ws])
+        b2, b3 = w[1][:, 64].contiguous(), w[2][:, 64].contiguous()
+        x, v, y, theta = Xb.cuda(), device(V), device(Y), w.reshape(-1).clone()
+        m, s, grad = torch.zeros_like(theta), torch.zeros_like(theta), torch.empty_like(theta)
+        part = device(np.zeros(L.acs_mlp_grad_bytes(n) // 4, np.float32))
+        lp = torch.empty((n + 127) // 128 * 4, device="cuda")
+        status = torch.zeros(8, dtype=torch.int32, device="cuda")
+        assert L.acs_mlp_train_step(x.data_ptr(), v.data_ptr(), y.data_ptr(), n, w5, b2.data_ptr(), b3.data_ptr(),
+                                    theta.data_ptr(), m.data_ptr(), s.data_ptr(), 1e-3, 1, 0.0, part.data_ptr(),
+                                    part.numel() * 4, lp.data_ptr(), grad.data_ptr(), status.data_ptr(), st) == 0
+        assert int(status[0].item()) == 0
+        out.append([t.cpu().numpy() for t in (grad, theta, lp)])
+    for a, b in zip(*out):
+        assert np.array_equal(a, b)
+    assert np.linalg.norm(out[0][0] - ref) <= 3e-2 * np.linalg.norm(ref)
+    assert abs(out[0][2].sum() - loss.item()) <= 1e-2 * loss.item()
