@@ -756,74 +756,6 @@ __device__ __forceinline__ bool dsf_excluded(const Eng& E, int32_t a, int32_t b)
   return false;
 }
 
-// Per-atom state of the list build: stencil ranges, FP32 screen and the exact FP64 decision.
-struct PairScan {
-  const Eng& E;
-  const RepDev& R;
-  int64_t i;
-  int c[3], lo[3], hi[3];
-  bool one[3];
-  float4 pi;
-  float lo_f, hi_f, Lf[3];
-  const float4* im;
-  int32_t* lst;
-
-  __device__ PairScan(const Eng& e, const RepDev& r, int64_t atom, int dst) : E(e), R(r), i(atom) {
-    cell_coords(E.cellid[i] - R.cellbase, R, c[0], c[1], c[2]);
-    im = E.img[dst];
-    pi = im[i];
-    const float rl2f = (float)R.rl2;
-    lo_f = rl2f * (1.0f - 1e-4f);
-    hi_f = rl2f * (1.0f + 1e-4f);
-    for (int d = 0; d < 3; ++d) {
-      Lf[d] = (float)R.L[d];
-      one[d] = R.nc[d] < 3;
-      lo[d] = one[d] ? 0 : -1;
-      hi[d] = one[d] ? 0 : 1;
-    }
-    lst = E.nbr + (i / E.G) * (int64_t)E.maxnb * E.G + (i % E.G);
-  }
-  __device__ int cell(int a, int b, int d) const {
-    const int n0 = wrapc(c[0] + a, R.nc[0]), n1 = wrapc(c[1] + b, R.nc[1]), n2 = wrapc(c[2] + d, R.nc[2]);
-    return R.cellbase + (n0 * R.nc[1] + n1) * R.nc[2] + n2;
-  }
-  // Exact decision for candidate k: the code to store, or -1. Band candidates use the FP64 filter; others
-  // are decided by the FP32 screen (with the FP32 wrap for one-cell axes).
-  __device__ int test(int k, int a, int b, int d) const {
-    const float4 pj = im[k];
-    float x = (pj.x - pi.x) + a * R.csf[0], y = (pj.y - pi.y) + b * R.csf[1], z = (pj.z - pi.z) + d * R.csf[2];
-    int w[3] = {0, 0, 0};
-    if (one[0]) { w[0] = x > 0.5f * Lf[0] ? 1 : (x < -0.5f * Lf[0] ? -1 : 0); x -= w[0] * Lf[0]; }
-    if (one[1]) { w[1] = y > 0.5f * Lf[1] ? 1 : (y < -0.5f * Lf[1] ? -1 : 0); y -= w[1] * Lf[1]; }
-    if (one[2]) { w[2] = z > 0.5f * Lf[2] ? 1 : (z < -0.5f * Lf[2] ? -1 : 0); z -= w[2] * Lf[2]; }
-    const float q = x * x + y * y + z * z;
-    if (!(q < hi_f)) return -1;
-    if (q <= lo_f) {
-      const int mx = one[0] ? -w[0] : a, my = one[1] ? -w[1] : b, mz = one[2] ? -w[2] : d;
-      return (mx + 1) + 3 * (my + 1) + 9 * (mz + 1);
-    }
-    double dx = sub(E.tmp_xa[3 * k], E.tmp_xa[3 * i]);
-    double dy = sub(E.tmp_xa[3 * k + 1], E.tmp_xa[3 * i + 1]);
-    double dz = sub(E.tmp_xa[3 * k + 2], E.tmp_xa[3 * i + 2]);
-    const int kx = dx > 0.5 * R.L[0] ? 1 : (dx < -0.5 * R.L[0] ? -1 : 0);
-    const int ky = dy > 0.5 * R.L[1] ? 1 : (dy < -0.5 * R.L[1] ? -1 : 0);
-    const int kz = dz > 0.5 * R.L[2] ? 1 : (dz < -0.5 * R.L[2] ? -1 : 0);
-    if (kx) dx = sub(dx, kx > 0 ? R.L[0] : -R.L[0]);
-    if (ky) dy = sub(dy, ky > 0 ? R.L[1] : -R.L[1]);
-    if (kz) dz = sub(dz, kz > 0 ? R.L[2] : -R.L[2]);
-    if (!(norm2(dx, dy, dz) < R.rl2)) return -1;
-    const int mx = one[0] ? -kx : a, my = one[1] ? -ky : b, mz = one[2] ? -kz : d;
-    return (mx + 1) + 3 * (my + 1) + 9 * (mz + 1);
-  }
-  __device__ void finish(int cnt) const {
-    E.nnb[i] = min(cnt, E.maxnb);
-    if (cnt > E.maxnb) {
-      atomicOr(&E.status->flags, ACS_FLAG_OVERFLOW);
-      atomicMax(&E.status->need_nbr, cnt);
-    }
-  }
-};
-
 // Grid-stride walk over the slots of the rebuild's flagged tiles (listed in phase P0 of this launch, read through
 // L2; padding slots excluded), calling f(s, r); with one replica, which is flagged whenever a rebuild runs, over
 // all its slots. An ensemble rebuild touches a few % of its slots, which this
@@ -844,32 +776,121 @@ __device__ __forceinline__ void for_flagged_slots(const Eng& E, int64_t gtid, in
   }
 }
 
-// The list of atom i built by one warp: the lanes take 32 candidates at a time, in stencil order and ascending
-// slot, and a ballot keeps the accepted ones in that order.
-template <bool EX>
-__device__ __forceinline__ void list_atom_warp(const Eng& E, const RepDev& R, int64_t i, int dst, int lane) {
-  PairScan ps(E, R, i, dst);
+// Exact decision for candidate k of atom i in the FP32 band around the list radius, at stencil offset (a, b, d): the code
+// to store, or -1. The reference's FP64 filter on the absolute positions, minimum image by comparison with box/2; on a
+// one-cell axis the code's shift is the image found here.
+__device__ __noinline__ int band_code(const Eng& E, const RepDev& R, int64_t i, int64_t k, int a, int b, int d) {
+  double dx = sub(E.tmp_xa[3 * k], E.tmp_xa[3 * i]);
+  double dy = sub(E.tmp_xa[3 * k + 1], E.tmp_xa[3 * i + 1]);
+  double dz = sub(E.tmp_xa[3 * k + 2], E.tmp_xa[3 * i + 2]);
+  const int kx = dx > 0.5 * R.L[0] ? 1 : (dx < -0.5 * R.L[0] ? -1 : 0);
+  const int ky = dy > 0.5 * R.L[1] ? 1 : (dy < -0.5 * R.L[1] ? -1 : 0);
+  const int kz = dz > 0.5 * R.L[2] ? 1 : (dz < -0.5 * R.L[2] ? -1 : 0);
+  if (kx) dx = sub(dx, kx > 0 ? R.L[0] : -R.L[0]);
+  if (ky) dy = sub(dy, ky > 0 ? R.L[1] : -R.L[1]);
+  if (kz) dz = sub(dz, kz > 0 ? R.L[2] : -R.L[2]);
+  if (!(norm2(dx, dy, dz) < R.rl2)) return -1;
+  const int mx = R.nc[0] < 3 ? -kx : a, my = R.nc[1] < 3 ? -ky : b, mz = R.nc[2] < 3 ? -kz : d;
+  return (mx + 1) + 3 * (my + 1) + 9 * (mz + 1);
+}
+
+// The list of atom i built by one warp: a ballot over 32 candidates keeps the accepted ones in stencil order and
+// ascending slot. The 27 stencil cells' slot ranges are read by 27 lanes at once and the candidates run through them as
+// one packed sequence, 32 kU loads in flight: a warp that walked cell after cell, each behind dependent loads from L2,
+// spent a small system's build waiting (864-atom argon 14.4 us of list build per rebuild, 10.4 now; 4096-ion NaCl, 27
+// cells of 152 ions, 94 us, 81 now). `shift`: 27 entries of shared memory for the image shifts, one per stencil cell.
+template <bool EX, int kU>
+__device__ __forceinline__ void list_atom_warp(const Eng& E, const RepDev& R, int64_t i, int dst, int lane,
+                                               float4* shift) {
+  const float4* __restrict__ im = E.img[dst];
+  const float4 pi = im[i];
+  const float rl2f = (float)R.rl2, lo_f = rl2f * (1.0f - 1e-4f), hi_f = rl2f * (1.0f + 1e-4f);
+  const bool one0 = R.nc[0] < 3, one1 = R.nc[1] < 3, one2 = R.nc[2] < 3, any_one = one0 || one1 || one2;
+  const float L0 = (float)R.L[0], L1 = (float)R.L[1], L2 = (float)R.L[2];
+  // lane st = 9 (a + 1) + 3 (b + 1) + (d + 1): its stencil cell's first slot, length and place P in the sequence
+  int sk0 = 0, slen = 0;
+  if (lane < 27) {
+    const int a = lane / 9 - 1, b = (lane / 3) % 3 - 1, d = lane % 3 - 1;
+    if ((!one0 || a == 0) && (!one1 || b == 0) && (!one2 || d == 0)) {
+      int c0, c1, c2;
+      cell_coords(E.cellid[i] - R.cellbase, R, c0, c1, c2);
+      const int n0 = wrapc(c0 + a, R.nc[0]), n1 = wrapc(c1 + b, R.nc[1]), n2 = wrapc(c2 + d, R.nc[2]);
+      const int p = E.crank[R.cellbase + (n0 * R.nc[1] + n1) * R.nc[2] + n2];
+      sk0 = E.start[p];
+      slen = E.start[p + 1] - sk0;
+    }
+    // the shift taken off this atom, and the entry's code
+    shift[lane] = make_float4(pi.x - a * R.csf[0], pi.y - b * R.csf[1], pi.z - d * R.csf[2],
+                              __int_as_float((a + 1) + 3 * (b + 1) + 9 * (d + 1)));
+  }
+  __syncwarp();
+  int incl = slen;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += y;
+  }
+  const int P = incl - slen, T = __shfl_sync(0xffffffffu, incl, 26);
+  const unsigned below = (1u << lane) - 1u;
+  int32_t* __restrict__ lst = E.nbr + (i / E.G) * (int64_t)E.maxnb * E.G + (i % E.G);
   int cnt = 0;
-  for (int a = ps.lo[0]; a <= ps.hi[0]; ++a)
-    for (int b = ps.lo[1]; b <= ps.hi[1]; ++b)
-      for (int d = ps.lo[2]; d <= ps.hi[2]; ++d) {
-        const int cc = ps.cell(a, b, d);
-        const int k0 = E.start[E.crank[cc]], k1 = E.start[E.crank[cc] + 1];
-        for (int base = k0; base < k1; base += 32) {
-          const int k = base + lane;
-          int code = -1;
-          if (k < k1 && k != i) code = ps.test(k, a, b, d);
-          const unsigned bal = __ballot_sync(0xffffffffu, code >= 0);
-          const int pos = cnt + __popc(bal & ((1u << lane) - 1u));
-          if (code >= 0 && pos < E.maxnb) {
-            uint32_t v = (uint32_t)k | ((uint32_t)code << kIdxBits);
-            if (EX && dsf_excluded(E, E.id[i], E.id[k])) v |= E.ex_bit;
-            ps.lst[(int64_t)pos * E.G] = (int32_t)v;
-          }
-          cnt += __popc(bal);
+  for (int pb = 0; pb < T; pb += 32 * kU) {
+    int k[kU], st[kU];
+    float4 pj[kU];
+#pragma unroll
+    for (int u = 0; u < kU; ++u) {
+      const int p = pb + 32 * u + lane;
+      const int pp = min(p, T - 1);
+      st[u] = 0;   // last stencil cell with P <= pp
+#pragma unroll
+      for (int step = 16; step > 0; step >>= 1) {
+        const int c = st[u] + step;
+        const int Pc = __shfl_sync(0xffffffffu, P, c < 27 ? c : 26);
+        if (c < 27 && Pc <= pp) st[u] = c;
+      }
+      k[u] = __shfl_sync(0xffffffffu, sk0, st[u]) + (pp - __shfl_sync(0xffffffffu, P, st[u]));
+      pj[u] = make_float4(3e30f, 3e30f, 3e30f, 0.f);   // past the end: r^2 overflows
+      if (p < T) pj[u] = im[k[u]];
+    }
+#pragma unroll
+    for (int u = 0; u < kU; ++u) {
+      if (pb + 32 * u >= T) break;
+      const float4 m = shift[st[u]];
+      float x = pj[u].x - m.x, y = pj[u].y - m.y, z = pj[u].z - m.z;
+      int code = __float_as_int(m.w);
+      const bool live = pb + 32 * u + lane < T && k[u] != i;
+      if (any_one && live) {   // the image of a one-cell axis is found per pair
+        if (one0) { const int w = x > 0.5f * L0 ? 1 : (x < -0.5f * L0 ? -1 : 0); x -= w * L0; code -= w; }
+        if (one1) { const int w = y > 0.5f * L1 ? 1 : (y < -0.5f * L1 ? -1 : 0); y -= w * L1; code -= 3 * w; }
+        if (one2) { const int w = z > 0.5f * L2 ? 1 : (z < -0.5f * L2 ? -1 : 0); z -= w * L2; code -= 9 * w; }
+      }
+      const float q = x * x + y * y + z * z;
+      bool in = live && q <= lo_f;
+      const bool band = live && q > lo_f && q < hi_f;
+      if (__any_sync(0xffffffffu, band)) {
+        if (band) {
+          code = band_code(E, R, i, k[u], st[u] / 9 - 1, (st[u] / 3) % 3 - 1, st[u] % 3 - 1);
+          in = code >= 0;
         }
       }
-  if (lane == 0) ps.finish(cnt);
+      const unsigned bal = __ballot_sync(0xffffffffu, in);
+      const int pos = cnt + __popc(bal & below);
+      if (in && pos < E.maxnb) {
+        uint32_t v = (uint32_t)k[u] | ((uint32_t)code << kIdxBits);
+        if (EX && dsf_excluded(E, E.id[i], E.id[k[u]])) v |= E.ex_bit;
+        lst[(int64_t)pos * E.G] = (int32_t)v;
+      }
+      cnt += __popc(bal);
+    }
+  }
+  if (lane == 0) {
+    E.nnb[i] = min(cnt, E.maxnb);
+    if (cnt > E.maxnb) {
+      atomicOr(&E.status->flags, ACS_FLAG_OVERFLOW);
+      atomicMax(&E.status->need_nbr, cnt);
+    }
+  }
+  __syncwarp();   // before the next atom's shifts
 }
 
 // Exact decision for a candidate in the FP32 band around the list radius, on a replica with >= 3 cells per
@@ -888,9 +909,10 @@ __device__ __noinline__ bool band_accept(const double* __restrict__ xa, int64_t 
 
 // Rebuild of flagged replicas and per-replica record reduction. Cooperative launch (all blocks resident);
 // every wait is bounded and reports ACS_FLAG_TIMEOUT instead of hanging. EX: the engine has DSF exclusions
-// (excluded pairs' list entries get the flag E.ex_bit).
-template <bool EX>
-__global__ void __launch_bounds__(256, 3) k_rebuild(Eng E, int dst, int rec, int rec_idx, int force_all) {
+// (excluded pairs' list entries get the flag E.ex_bit). ATOMS: the lists a warp per atom (engines of 8 and more threads
+// per atom, whose grids leave registers to spare), else a warp per cell.
+template <bool EX, bool ATOMS>
+__global__ void __launch_bounds__(256, ATOMS ? 2 : 3) k_rebuild(Eng E, int dst, int rec, int rec_idx, int force_all) {
   __shared__ unsigned char fl[kMaxRep];
   __shared__ int any_s;
   if (threadIdx.x == 0) any_s = 0;
@@ -1147,7 +1169,8 @@ __global__ void __launch_bounds__(256, 3) k_rebuild(Eng E, int dst, int rec, int
   // minus the wrap (1 cell per edge). Entries are in stencil order, ascending slot within a cell, however
   // the work is split: a warp per atom when the pair kernel runs >= 8 threads per atom (small systems), else a
   // warp per home cell, and a warp per atom for replicas with a one-cell axis.
-  if (E.tpa >= 8) {
+  __shared__ float4 bufp[8][64];
+  if (ATOMS) {
     const int64_t gw = gtid >> 5, nw = gstride >> 5;
     const int lane = threadIdx.x & 31;
     for (int64_t i = gw; i < E.S; i += nw) {
@@ -1155,7 +1178,7 @@ __global__ void __launch_bounds__(256, 3) k_rebuild(Eng E, int dst, int rec, int
       if (!fl[r]) continue;
       const RepDev& R = E.rep[r];
       if (i - R.atom0 >= R.n) continue;
-      list_atom_warp<EX>(E, R, i, dst, lane);
+      list_atom_warp<EX, 4>(E, R, i, dst, lane, bufp[threadIdx.x >> 5]);
     }
   } else {
     // Replicas with >= 3 cells on every axis: a warp per home cell (a warp takes the next of the flagged
@@ -1169,7 +1192,6 @@ __global__ void __launch_bounds__(256, 3) k_rebuild(Eng E, int dst, int rec, int
     // FP64 band decision branches.
     // home atoms' negated coordinates, one array per axis: two adjacent home atoms load as one packed FP32 pair
     __shared__ __align__(8) float hnx[8][32], hny[8][32], hnz[8][32];
-    __shared__ float4 bufp[8][64];
     __shared__ uint32_t bufk[8][64];
     __shared__ int selfpos[8][32];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
@@ -1384,7 +1406,7 @@ __global__ void __launch_bounds__(256, 3) k_rebuild(Eng E, int dst, int rec, int
       for (int q = q0; q < q1; ++q) {
         while (r + 1 < E.R && __ldcg(E.fsmall + r + 1) <= q) ++r;
         const RepDev& R = E.rep[r];
-        list_atom_warp<EX>(E, R, R.atom0 + (q - __ldcg(E.fsmall + r)), dst, lane);
+        list_atom_warp<EX, 1>(E, R, R.atom0 + (q - __ldcg(E.fsmall + r)), dst, lane, bufp[wib]);
       }
     }
   }
@@ -2001,6 +2023,12 @@ int launch_correction(acs_engine* e, int src, cudaStream_t s) {
   return acs_mlp_forward(e->c_X, e->c_V, e->E.S, e->c_w5, e->c_b2, e->c_b3, e->c_scale, e->c_F, e->c_status, s);
 }
 
+using RebuildKernel = void (*)(Eng, int, int, int, int);
+RebuildKernel rebuild_kernel(const Eng& E) {
+  if (E.tpa >= 8) return E.ex_bit ? k_rebuild<true, true> : k_rebuild<false, true>;
+  return E.ex_bit ? k_rebuild<true, false> : k_rebuild<false, false>;
+}
+
 int launch_rebuild(acs_engine* e, int dst, int rec, int rec_idx, int force_all, cudaStream_t s) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(e->coop_blocks);
@@ -2011,8 +2039,7 @@ int launch_rebuild(acs_engine* e, int dst, int rec, int rec_idx, int force_all, 
   attr[0].val.cooperative = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  cudaError_t err = e->E.ex_bit ? cudaLaunchKernelEx(&cfg, k_rebuild<true>, e->E, dst, rec, rec_idx, force_all)
-                                 : cudaLaunchKernelEx(&cfg, k_rebuild<false>, e->E, dst, rec, rec_idx, force_all);
+  cudaError_t err = cudaLaunchKernelEx(&cfg, rebuild_kernel(e->E), e->E, dst, rec, rec_idx, force_all);
   return err == cudaSuccess ? ACS_OK : ACS_ERR_CUDA;
 }
 
@@ -2237,8 +2264,7 @@ int acs_engine_create(const acs_engine_config* cfg, void* mem, size_t bytes, acs
   ok = ok && cudaMemset(E.rec_bath, 0, 8 * (size_t)E.rec_cap * E.R) == cudaSuccess;
   int sms = 0, per_sm = 0;
   ok = ok && cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, e->dev) == cudaSuccess;
-  ok = ok && cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, E.ex_bit ? k_rebuild<true> : k_rebuild<false>,
-                                                           256, 0) == cudaSuccess;
+  ok = ok && cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, rebuild_kernel(E), 256, 0) == cudaSuccess;
   if (!ok || per_sm < 1) {
     delete e;
     return ACS_ERR_CUDA;
