@@ -97,8 +97,9 @@ struct Eng {
   int32_t ncc;
   int32_t *cc_rep, *cc_c0, *cc_n, *cc_sum;
   double *xa, *tmp_xa, *tmp_v;
-  int32_t *tmp_cell, *tmp_id, *tmp_sp, *newcell, *perm, *perm2;
-  int32_t *count, *start, *cursor;
+  int32_t *tmp_cell, *tmp_id, *tmp_sp, *newcell, *perm, *place;
+  int32_t *count, *start;
+  int32_t scan_by_replica;       // every replica's cells are few chunks: a block scans a replica
   // slot order of cells: cells' atoms occupy consecutive slots in the order given by crank (cell id -> position,
   // both global over replicas); start[] is indexed by position, so the atoms of cell c are the slots
   // [start[crank[c]], start[crank[c] + 1]). cell_at is the inverse (position -> cell id).
@@ -908,6 +909,10 @@ __device__ __noinline__ bool band_accept(const double* __restrict__ xa, int64_t 
 }
 
 // Rebuild of flagged replicas and per-replica record reduction. Cooperative launch (all blocks resident);
+// each of a rebuild's phases ends in a grid barrier, 2 to 3 us with its first loads, which is what small systems'
+// rebuilds cost: five barriers before the list build with one replica, a sixth for the tile list of several (ten
+// before counts were left clear for the next rebuild, the scan and the in-cell order taken in one phase each: 864-atom
+// argon 36 -> 19 us of a rebuild's phases, 48 replicas 9.3 -> 8.5 ms for 50 steps).
 // every wait is bounded and reports ACS_FLAG_TIMEOUT instead of hanging. EX: the engine has DSF exclusions
 // (excluded pairs' list entries get the flag E.ex_bit). ATOMS: the lists a warp per atom (engines of 8 and more threads
 // per atom, whose grids leave registers to spare), else a warp per cell.
@@ -989,7 +994,6 @@ __global__ void __launch_bounds__(256, ATOMS ? 2 : 3) k_rebuild(Eng E, int dst, 
       E.fcell[E.R + 1] = 0;   // the list build's cell counter
       E.fsmall[E.R] = total_s;
       E.fsmall[E.R + 1] = 0;  // and its atom-unit counter
-      E.ftile[E.S >> 5] = 0;  // the flagged-tile count
     }
   }
 #define PHASE(k)                                                  \
@@ -998,17 +1002,9 @@ __global__ void __launch_bounds__(256, ATOMS ? 2 : 3) k_rebuild(Eng E, int dst, 
     atomicAdd(&E.phase_ns[k], t_now - t_prev);                    \
     t_prev = t_now;                                               \
   }
-  if (!grid_sync(E.bar, E.status, E.spin_limit)) return;
-  PHASE(1);
-
-  // P0: clear counters of flagged replicas' cells; list the flagged replicas' tiles (a warp appends its tiles
-  // with one atomic), which the slot phases then walk instead of skipping the unflagged replicas' slots
-  for (int64_t c = gtid; c < E.C; c += gstride) {
-    if (fl[E.cell_rep[c]]) {
-      E.count[c] = 0;
-      E.cursor[c] = 0;
-    }
-  }
+  // P0, several replicas: list the flagged replicas' tiles (a warp appends its tiles with one atomic), which the slot
+  // phases then walk instead of skipping the unflagged replicas' slots. The list's count and the cells' counts are zero
+  // when a rebuild starts: the list build and the commit of the last one cleared them.
   if (E.R > 1) {
     const int lane = threadIdx.x & 31;
     const int64_t T = E.S >> 5;
@@ -1021,10 +1017,10 @@ __global__ void __launch_bounds__(256, ATOMS ? 2 : 3) k_rebuild(Eng E, int dst, 
       base = __shfl_sync(0xffffffffu, base, 0);
       if (f) E.ftile[base + __popc(bal & ((1u << lane) - 1u))] = (int32_t)t;
     }
+    if (!grid_sync(E.bar, E.status, E.spin_limit)) return;
   }
-  if (!grid_sync(E.bar, E.status, E.spin_limit)) return;
-  PHASE(2);
-  // P1: absolute wrapped positions and new cells
+  PHASE(1);
+  // P1: absolute wrapped positions, new cells, arrival number within the cell
   for_flagged_slots(E, gtid, gstride, [&](int64_t s, int r) {
     const RepDev& R = E.rep[r];
     int c0, c1, c2;
@@ -1048,90 +1044,118 @@ __global__ void __launch_bounds__(256, ATOMS ? 2 : 3) k_rebuild(Eng E, int dst, 
     }
     const int c = R.cellbase + (nc3[0] * R.nc[1] + nc3[1]) * R.nc[2] + nc3[2];
     E.newcell[s] = c;
-    atomicAdd(&E.count[c], 1);
+    E.place[s] = atomicAdd(&E.count[c], 1);
   });
   if (!grid_sync(E.bar, E.status, E.spin_limit)) return;
   PHASE(3);
-  // P2: exclusive scan of cell counts -> slot starts, in fixed 1024-cell chunks: (a) chunk-local scans,
-  // (b) per-replica prefix of chunk totals (also: sentinel, clear flag, count the rebuild), (c) offsets.
-  for (int c = blockIdx.x; c < E.ncc; c += gridDim.x) {
-    if (!fl[E.cc_rep[c]]) continue;
-    const int c0 = E.cc_c0[c], nc = E.cc_n[c];
-    int v[4], sum = 0;
+  // P2: exclusive scan of cell counts -> slot starts; sentinel, clear flag, count the rebuild. Where every replica is a
+  // few chunks of 1024 cells a block scans a replica, chunk after chunk; else in three phases: (a) chunk-local scans,
+  // (b) per-replica prefix of chunk totals, (c) offsets. (Each phase's barrier is about 2 us.)
+  if (E.scan_by_replica) {
+    for (int r = blockIdx.x; r < E.R; r += gridDim.x) {
+      if (!fl[r]) continue;
+      const RepDev& R = E.rep[r];
+      int carry = (int)R.atom0;
+      for (int q0 = 0; q0 < R.ncells; q0 += kCellChunk) {
+        const int c0 = R.cellbase + q0, nc = min(kCellChunk, R.ncells - q0);
+        int v[4], sum = 0;
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int idx = 4 * threadIdx.x + q;
-      v[q] = idx < nc ? E.count[E.cell_at[c0 + idx]] : 0;
-      sum += v[q];
-    }
-    int total;
-    int ex = block_scan_excl(sum, &total);
+        for (int q = 0; q < 4; ++q) {
+          const int idx = 4 * threadIdx.x + q;
+          v[q] = idx < nc ? E.count[E.cell_at[c0 + idx]] : 0;
+          sum += v[q];
+        }
+        int total;
+        int ex = carry + block_scan_excl(sum, &total);
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int idx = 4 * threadIdx.x + q;
-      if (idx < nc) E.start[c0 + idx] = ex;
-      ex += v[q];
+        for (int q = 0; q < 4; ++q) {
+          const int idx = 4 * threadIdx.x + q;
+          if (idx < nc) E.start[c0 + idx] = ex;
+          ex += v[q];
+        }
+        carry += total;
+      }
+      if (threadIdx.x == 0) {
+        E.start[R.cellbase + R.ncells] = (int32_t)(R.atom0 + R.n);
+        E.flag[r] = 0;
+        atomicAdd(&E.status->rebuilds, 1);
+      }
     }
-    if (threadIdx.x == 0) E.cc_sum[c] = total;
-  }
-  if (!grid_sync(E.bar, E.status, E.spin_limit)) return;
-  PHASE(4);
-  // (b) a block per flagged replica scans its chunk totals (exclusive, from the replica's first slot)
-  for (int r = blockIdx.x; r < E.R; r += gridDim.x) {
-    if (!fl[r]) continue;
-    const RepDev& R = E.rep[r];
-    int carry = 0;
-    for (int c0 = 0; c0 < R.ncc; c0 += blockDim.x) {
-      const int c = c0 + (int)threadIdx.x;
-      const int t = c < R.ncc ? E.cc_sum[R.cc0 + c] : 0;
+    if (!grid_sync(E.bar, E.status, E.spin_limit)) return;
+  } else {
+    for (int c = blockIdx.x; c < E.ncc; c += gridDim.x) {
+      if (!fl[E.cc_rep[c]]) continue;
+      const int c0 = E.cc_c0[c], nc = E.cc_n[c];
+      int v[4], sum = 0;
+  #pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int idx = 4 * threadIdx.x + q;
+        v[q] = idx < nc ? E.count[E.cell_at[c0 + idx]] : 0;
+        sum += v[q];
+      }
       int total;
-      const int ex = block_scan_excl(t, &total);
-      if (c < R.ncc) E.cc_sum[R.cc0 + c] = (int32_t)(R.atom0 + carry + ex);
-      carry += total;
+      int ex = block_scan_excl(sum, &total);
+  #pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int idx = 4 * threadIdx.x + q;
+        if (idx < nc) E.start[c0 + idx] = ex;
+        ex += v[q];
+      }
+      if (threadIdx.x == 0) E.cc_sum[c] = total;
     }
-    if (threadIdx.x == 0) {
-      E.start[R.cellbase + R.ncells] = (int32_t)(R.atom0 + R.n);
-      E.flag[r] = 0;
-      atomicAdd(&E.status->rebuilds, 1);
+    if (!grid_sync(E.bar, E.status, E.spin_limit)) return;
+    PHASE(4);
+    // (b) a block per flagged replica scans its chunk totals (exclusive, from the replica's first slot)
+    for (int r = blockIdx.x; r < E.R; r += gridDim.x) {
+      if (!fl[r]) continue;
+      const RepDev& R = E.rep[r];
+      int carry = 0;
+      for (int c0 = 0; c0 < R.ncc; c0 += blockDim.x) {
+        const int c = c0 + (int)threadIdx.x;
+        const int t = c < R.ncc ? E.cc_sum[R.cc0 + c] : 0;
+        int total;
+        const int ex = block_scan_excl(t, &total);
+        if (c < R.ncc) E.cc_sum[R.cc0 + c] = (int32_t)(R.atom0 + carry + ex);
+        carry += total;
+      }
+      if (threadIdx.x == 0) {
+        E.start[R.cellbase + R.ncells] = (int32_t)(R.atom0 + R.n);
+        E.flag[r] = 0;
+        atomicAdd(&E.status->rebuilds, 1);
+      }
     }
+    if (!grid_sync(E.bar, E.status, E.spin_limit)) return;
+    PHASE(5);
+    for (int c = blockIdx.x; c < E.ncc; c += gridDim.x) {
+      if (!fl[E.cc_rep[c]]) continue;
+      const int c0 = E.cc_c0[c], nc = E.cc_n[c], add_v = E.cc_sum[c];
+      for (int idx = threadIdx.x; idx < nc; idx += blockDim.x) E.start[c0 + idx] += add_v;
+    }
+    if (!grid_sync(E.bar, E.status, E.spin_limit)) return;
   }
-  if (!grid_sync(E.bar, E.status, E.spin_limit)) return;
-  PHASE(5);
-  for (int c = blockIdx.x; c < E.ncc; c += gridDim.x) {
-    if (!fl[E.cc_rep[c]]) continue;
-    const int c0 = E.cc_c0[c], nc = E.cc_n[c], add_v = E.cc_sum[c];
-    for (int idx = threadIdx.x; idx < nc; idx += blockDim.x) E.start[c0 + idx] += add_v;
-  }
-  if (!grid_sync(E.bar, E.status, E.spin_limit)) return;
   PHASE(6);
   // P3: scatter old slots to new slots
   for_flagged_slots(E, gtid, gstride, [&](int64_t s, int) {
-    const int c = E.newcell[s];
-    E.perm[E.start[E.crank[c]] + atomicAdd(&E.cursor[c], 1)] = (int32_t)s;
+    E.perm[E.start[E.crank[E.newcell[s]]] + E.place[s]] = (int32_t)s;
   });
   if (!grid_sync(E.bar, E.status, E.spin_limit)) return;
   PHASE(7);
-  // P3b: deterministic order inside each cell: every atom's rank among its cell's atoms by old slot
-  for_flagged_slots(E, gtid, gstride, [&](int64_t k, int) {
-    const int v = E.perm[k];
-    const int c = E.newcell[v];
+  // P4: gather into new order, deterministic inside each cell: every atom's rank among its cell's atoms by old slot is
+  // its place
+  for_flagged_slots(E, gtid, gstride, [&](int64_t q, int) {
+    const int o = E.perm[q];
+    const int c = E.newcell[o];
     const int a0 = E.start[E.crank[c]], a1 = E.start[E.crank[c] + 1];
     int rank = 0;
-    for (int a = a0; a < a1; ++a) rank += (E.perm[a] < v);
-    E.perm2[a0 + rank] = v;
-  });
-  if (!grid_sync(E.bar, E.status, E.spin_limit)) return;
-  PHASE(8);
-  // P4: gather into new order
-  for_flagged_slots(E, gtid, gstride, [&](int64_t k, int) {
-    const int o = E.perm2[k];
-    E.tmp_cell[k] = E.newcell[o];
+    for (int a = a0; a < a1; ++a) rank += (E.perm[a] < o);
+    const int64_t k = a0 + rank;
+    E.tmp_cell[k] = c;
     E.tmp_id[k] = E.id[o];
     E.tmp_sp[k] = E.sp[o];
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
-      E.tmp_xa[3 * k + d] = E.xa[3 * o + d];
-      E.tmp_v[3 * k + d] = E.v[3 * o + d];
+      E.tmp_xa[3 * k + d] = E.xa[3 * (int64_t)o + d];
+      E.tmp_v[3 * k + d] = E.v[3 * (int64_t)o + d];
     }
   });
   if (!grid_sync(E.bar, E.status, E.spin_limit)) return;
@@ -1158,8 +1182,11 @@ __global__ void __launch_bounds__(256, ATOMS ? 2 : 3) k_rebuild(Eng E, int dst, 
     for (int d = 0; d < 3; ++d) E.v[3 * k + d] = E.tmp_v[3 * k + d];
     E.img[dst][k] = make_img(ux, uy, uz, E.tmp_sp[k]);
   });
+  for (int64_t c = gtid; c < E.C; c += gstride)   // for the next rebuild
+    if (fl[E.cell_rep[c]]) E.count[c] = 0;
   if (!grid_sync(E.bar, E.status, E.spin_limit)) return;
   PHASE(10);
+  if (gtid == 0) E.ftile[E.S >> 5] = 0;   // the tile list has been walked for the last time
   // P6: neighbour lists in one pass over the 27-cell stencil. Each candidate's r^2 is first computed in
   // FP32 from the new images (relative error ~1e-6): outside rl^2 (1 + 1e-4) it is rejected, inside
   // rl^2 (1 - 1e-4) accepted; only the band between is decided by the reference's FP64 filter. So the
@@ -1863,31 +1890,30 @@ Layout make_layout(int32_t R, int64_t S, int32_t T, int32_t C, int32_t NCH, int3
   L.add(4 * (size_t)S);                      // 26 perm
   L.add(4 * (size_t)C);                      // 27 count
   L.add(4 * (size_t)C);                      // 28 start
-  L.add(4 * (size_t)C);                      // 29 cursor
-  L.add(8 * (size_t)NG * kRecW);             // 30 partials (one row per atom group)
-  L.add(8 * (size_t)NCH * kRecW);            // 31 chunk partials
-  L.add(8 * (size_t)rec_cap * R * kRecW);    // 32 records
-  L.add(sizeof(acs_dev_status));             // 33 status
-  L.add(16);                                 // 34 barrier
-  L.add(8 * (size_t)R);                      // 35 src0
-  L.add(4 * (size_t)NCC);                    // 36 cc_rep
-  L.add(4 * (size_t)NCC);                    // 37 cc_c0
-  L.add(4 * (size_t)NCC);                    // 38 cc_n
-  L.add(4 * (size_t)NCC);                    // 39 cc_sum
-  L.add(8 * 16);                             // 40 phase timers
-  L.add(4 * (size_t)S);                      // 41 perm2
-  L.add(8);                                  // 42 Langevin O-step counter
-  L.add(8 * (size_t)NG);                     // 43 Nose-Hoover group partials
-  L.add(8 * (size_t)NCH);                    // 44 Nose-Hoover chunk partials
-  L.add(8 * 8 * (size_t)R);                  // 45 Nose-Hoover state
-  L.add(8 * (size_t)rec_cap * R);            // 46 bath-energy records
-  L.add(4 * ((size_t)R + 2));                // 47 flagged-cell prefix of a rebuild, list-build cell counter
-  L.add(4 * ((size_t)n_ex_ids + 1));         // 48 DSF exclusions: CSR starts by atom id
-  L.add(4 * ((size_t)n_ex + 1));             // 49 DSF exclusions: excluded ids
-  L.add(4 * (size_t)C);                      // 50 crank (cell id -> slot-order position)
-  L.add(4 * (size_t)C);                      // 51 cell_at (position -> cell id)
-  L.add(4 * ((size_t)R + 2));                // 52 flagged one-cell-axis atoms prefix, list-build unit counter
-  L.add(4 * ((size_t)T + 1));                // 53 flagged tiles of a rebuild and their count
+  L.add(8 * (size_t)NG * kRecW);             // 29 partials (one row per atom group)
+  L.add(8 * (size_t)NCH * kRecW);            // 30 chunk partials
+  L.add(8 * (size_t)rec_cap * R * kRecW);    // 31 records
+  L.add(sizeof(acs_dev_status));             // 32 status
+  L.add(16);                                 // 33 barrier
+  L.add(8 * (size_t)R);                      // 34 src0
+  L.add(4 * (size_t)NCC);                    // 35 cc_rep
+  L.add(4 * (size_t)NCC);                    // 36 cc_c0
+  L.add(4 * (size_t)NCC);                    // 37 cc_n
+  L.add(4 * (size_t)NCC);                    // 38 cc_sum
+  L.add(8 * 16);                             // 39 phase timers
+  L.add(4 * (size_t)S);                      // 40 place (arrival number of a slot's atom in its new cell)
+  L.add(8);                                  // 41 Langevin O-step counter
+  L.add(8 * (size_t)NG);                     // 42 Nose-Hoover group partials
+  L.add(8 * (size_t)NCH);                    // 43 Nose-Hoover chunk partials
+  L.add(8 * 8 * (size_t)R);                  // 44 Nose-Hoover state
+  L.add(8 * (size_t)rec_cap * R);            // 45 bath-energy records
+  L.add(4 * ((size_t)R + 2));                // 46 flagged-cell prefix of a rebuild, list-build cell counter
+  L.add(4 * ((size_t)n_ex_ids + 1));         // 47 DSF exclusions: CSR starts by atom id
+  L.add(4 * ((size_t)n_ex + 1));             // 48 DSF exclusions: excluded ids
+  L.add(4 * (size_t)C);                      // 49 crank (cell id -> slot-order position)
+  L.add(4 * (size_t)C);                      // 50 cell_at (position -> cell id)
+  L.add(4 * ((size_t)R + 2));                // 51 flagged one-cell-axis atoms prefix, list-build unit counter
+  L.add(4 * ((size_t)T + 1));                // 52 flagged tiles of a rebuild and their count
   return L;
 }
 
@@ -2151,33 +2177,35 @@ int acs_engine_create(const acs_engine_config* cfg, void* mem, size_t bytes, acs
   E.perm = (int32_t*)(b + L.off[26]);
   E.count = (int32_t*)(b + L.off[27]);
   E.start = (int32_t*)(b + L.off[28]);
-  E.cursor = (int32_t*)(b + L.off[29]);
-  E.partials = (double*)(b + L.off[30]);
-  E.chunk_part = (double*)(b + L.off[31]);
-  E.rec = (double*)(b + L.off[32]);
-  E.status = (acs_dev_status*)(b + L.off[33]);
-  E.bar = (unsigned int*)(b + L.off[34]);
-  e->src0_dev = (int64_t*)(b + L.off[35]);
+  E.partials = (double*)(b + L.off[29]);
+  E.chunk_part = (double*)(b + L.off[30]);
+  E.rec = (double*)(b + L.off[31]);
+  E.status = (acs_dev_status*)(b + L.off[32]);
+  E.bar = (unsigned int*)(b + L.off[33]);
+  e->src0_dev = (int64_t*)(b + L.off[34]);
   E.ncc = NCC;
-  E.cc_rep = (int32_t*)(b + L.off[36]);
-  E.cc_c0 = (int32_t*)(b + L.off[37]);
-  E.cc_n = (int32_t*)(b + L.off[38]);
-  E.cc_sum = (int32_t*)(b + L.off[39]);
-  E.phase_ns = (unsigned long long*)(b + L.off[40]);
-  E.perm2 = (int32_t*)(b + L.off[41]);
-  E.octr = (unsigned long long*)(b + L.off[42]);
-  E.nh_part = (double*)(b + L.off[43]);
-  E.nh_chunk = (double*)(b + L.off[44]);
-  E.nh_st = (double*)(b + L.off[45]);
-  E.rec_bath = (double*)(b + L.off[46]);
-  E.fcell = (int32_t*)(b + L.off[47]);
+  E.scan_by_replica = 1;
+  for (const RepDev& R : e->reps)
+    if (R.ncc > 4) E.scan_by_replica = 0;
+  E.cc_rep = (int32_t*)(b + L.off[35]);
+  E.cc_c0 = (int32_t*)(b + L.off[36]);
+  E.cc_n = (int32_t*)(b + L.off[37]);
+  E.cc_sum = (int32_t*)(b + L.off[38]);
+  E.phase_ns = (unsigned long long*)(b + L.off[39]);
+  E.place = (int32_t*)(b + L.off[40]);
+  E.octr = (unsigned long long*)(b + L.off[41]);
+  E.nh_part = (double*)(b + L.off[42]);
+  E.nh_chunk = (double*)(b + L.off[43]);
+  E.nh_st = (double*)(b + L.off[44]);
+  E.rec_bath = (double*)(b + L.off[45]);
+  E.fcell = (int32_t*)(b + L.off[46]);
   E.n_ex_ids = cfg->n_ex_ids;
-  E.ex_start = (const int32_t*)(b + L.off[48]);
-  E.ex_ids = (const int32_t*)(b + L.off[49]);
-  E.crank = (int32_t*)(b + L.off[50]);
-  E.cell_at = (int32_t*)(b + L.off[51]);
-  E.fsmall = (int32_t*)(b + L.off[52]);
-  E.ftile = (int32_t*)(b + L.off[53]);
+  E.ex_start = (const int32_t*)(b + L.off[47]);
+  E.ex_ids = (const int32_t*)(b + L.off[48]);
+  E.crank = (int32_t*)(b + L.off[49]);
+  E.cell_at = (int32_t*)(b + L.off[50]);
+  E.fsmall = (int32_t*)(b + L.off[51]);
+  E.ftile = (int32_t*)(b + L.off[52]);
   E.ex_bit = cfg->n_ex_ids > 0 ? kExBit : 0u;
   E.jmask = cfg->n_ex_ids > 0 ? kExBit - 1u : kIdxMask;
   E.thermo = cfg->thermo.kind;
@@ -2251,6 +2279,8 @@ int acs_engine_create(const acs_engine_config* cfg, void* mem, size_t bytes, acs
   ok = ok && cudaMemcpy(E.cc_c0, cc_c0.data(), 4 * (size_t)NCC, cudaMemcpyHostToDevice) == cudaSuccess;
   ok = ok && cudaMemcpy(E.cc_n, cc_n.data(), 4 * (size_t)NCC, cudaMemcpyHostToDevice) == cudaSuccess;
   ok = ok && cudaMemset(E.nnb, 0, 4 * (size_t)S) == cudaSuccess;
+  ok = ok && cudaMemset(E.count, 0, 4 * (size_t)C) == cudaSuccess;
+  ok = ok && cudaMemset(E.ftile + T, 0, 4) == cudaSuccess;
   ok = ok && cudaMemset(E.phase_ns, 0, 8 * 16) == cudaSuccess;
   ok = ok && cudaMemset(E.octr, 0, 8) == cudaSuccess;
   ok = ok && cudaMemset(E.nh_st, 0, 8 * 8 * (size_t)E.R) == cudaSuccess;
@@ -2373,9 +2403,12 @@ int acs_engine_status(acs_engine* e, acs_dev_status* out, int clear, void* strea
     if (cudaMemcpyAsync(e->E.status, &z, sizeof(z), cudaMemcpyHostToDevice, s) != cudaSuccess ||
         cudaStreamSynchronize(s) != cudaSuccess)
       return ACS_ERR_CUDA;
-    // a barrier that timed out leaves its arrival count behind: start the next launch from a clean barrier
+    // a barrier that timed out leaves its arrival count behind, and a rebuild that it ended its cells' and tiles' counts:
+    // start the next launch from clean ones
     if ((out->flags & ACS_FLAG_TIMEOUT) &&
-        (cudaMemsetAsync(e->E.bar, 0, 16, s) != cudaSuccess || cudaStreamSynchronize(s) != cudaSuccess))
+        (cudaMemsetAsync(e->E.bar, 0, 16, s) != cudaSuccess ||
+         cudaMemsetAsync(e->E.count, 0, 4 * (size_t)e->E.C, s) != cudaSuccess ||
+         cudaMemsetAsync(e->E.ftile + e->E.T, 0, 4, s) != cudaSuccess || cudaStreamSynchronize(s) != cudaSuccess))
       return ACS_ERR_CUDA;
   }
   return ACS_OK;

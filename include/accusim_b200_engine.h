@@ -129,8 +129,8 @@ int acs_engine_launch_info(acs_engine* e, int32_t* step_blocks, int32_t* coop_bl
  * out_ms = {step-kernel ms total, list-maintenance ms total, step launches, list-maintenance launches}. */
 int acs_engine_run_timed(acs_engine* e, int32_t steps, int32_t record_every, float* out_ms, void* stream);
 /* Accumulated wall time (ns, device global timer, block 0's view) of the list-maintenance phases:
- * [1] flag read, [2] clear, [3] bin, [4..6] scan, [7] scatter, [8] in-cell sort, [9] gather, [10] commit,
- * [15] list build (block 0 share). Synchronous. */
+ * [1] flag read and tile list, [3] bin, [4..6] scan (all in [6] where a block scans a replica), [7] scatter, [9] in-cell
+ * sort and gather, [10] commit, [15] list build (block 0 share); the others stay 0. Synchronous. */
 int acs_engine_phase_times(acs_engine* e, unsigned long long* out16, int clear);
 /* Learned force correction (no counterpart in the reference): when enabled, every force evaluation first
  * computes the radial descriptors of all slots from the engine's images and lists (radius params6[3] <= list
