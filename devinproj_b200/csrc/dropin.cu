@@ -43,16 +43,21 @@ __device__ __forceinline__ int bin1(double x, double lo, double span, int nc) {
   return (int)t;
 }
 
+__device__ __forceinline__ int cell_index(const double* __restrict__ pos, int64_t i, const GridDev& g) {
+  const int c0 = bin1(pos[3 * i + 0], g.lo[0], g.span[0], g.nc[0]);
+  const int c1 = bin1(pos[3 * i + 1], g.lo[1], g.span[1], g.nc[1]);
+  const int c2 = bin1(pos[3 * i + 2], g.lo[2], g.span[2], g.nc[2]);
+  return (c0 * g.nc[1] + c1) * g.nc[2] + c2;
+}
+
+// place: the atom's arrival number in its cell.
 __global__ void k_bin(const double* __restrict__ pos, int64_t n, GridDev g, int32_t* __restrict__ cell_of,
-                      int32_t* __restrict__ count) {
+                      int32_t* __restrict__ place, int32_t* __restrict__ count) {
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  int c0 = bin1(pos[3 * i + 0], g.lo[0], g.span[0], g.nc[0]);
-  int c1 = bin1(pos[3 * i + 1], g.lo[1], g.span[1], g.nc[1]);
-  int c2 = bin1(pos[3 * i + 2], g.lo[2], g.span[2], g.nc[2]);
-  int c = (c0 * g.nc[1] + c1) * g.nc[2] + c2;
+  const int c = cell_index(pos, i, g);
   cell_of[i] = c;
-  atomicAdd(&count[c], 1);
+  place[i] = atomicAdd(&count[c], 1);
 }
 
 // Three-phase exclusive scan over int32 (chunk of 4096 per 1024-thread block).
@@ -130,13 +135,55 @@ __global__ void k_scan_add(int32_t* __restrict__ out, int64_t len, const int32_t
     if (base + k < len) out[base + k] += add_v;
 }
 
-__global__ void k_scatter(const int32_t* __restrict__ cell_of, int64_t n, const int32_t* __restrict__ start,
-                          int32_t* __restrict__ cursor, int32_t* __restrict__ cell_atoms) {
+__global__ void k_scatter(const int32_t* __restrict__ cell_of, const int32_t* __restrict__ place, int64_t n,
+                          const int32_t* __restrict__ start, int32_t* __restrict__ unsorted) {
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  int c = cell_of[i];
-  int slot = atomicAdd(&cursor[c], 1);
-  cell_atoms[start[c] + slot] = (int32_t)i;
+  if (i < n) unsorted[start[cell_of[i]] + place[i]] = (int32_t)i;
+}
+
+// Counting, scan and scatter of up to kBinAtoms atoms into fewer than kBinCells cells by one block, the counts in shared
+// memory: in small systems the launches of the general path (six and a clear) are most of its time. Whole list build of 864
+// atoms 41 -> 23 us, 4096 ions 54 -> 37, 8000 ions 74 -> 56 (one block 11 us against 13 in seven launches).
+constexpr int kBinAtoms = 8192, kBinCells = 8192;
+__global__ void __launch_bounds__(1024) k_bin_block(const double* __restrict__ pos, int n,
+                                                    const __grid_constant__ GridDev g, int nc,
+                                                    int32_t* __restrict__ cell_of, int32_t* __restrict__ start,
+                                                    int32_t* __restrict__ unsorted) {
+  constexpr int kA = kBinAtoms / 1024, kC = kBinCells / 1024;
+  __shared__ int count[kBinCells];
+  for (int c = threadIdx.x; c < kBinCells; c += 1024) count[c] = 0;
+  __syncthreads();
+  int cell[kA], place[kA];
+#pragma unroll
+  for (int q = 0; q < kA; ++q) {
+    const int i = threadIdx.x + 1024 * q;
+    cell[q] = i < n ? cell_index(pos, i, g) : 0;
+    if (i < n) {
+      cell_of[i] = cell[q];
+      place[q] = atomicAdd(&count[cell[q]], 1);
+    }
+  }
+  __syncthreads();
+  int v[kC], sum = 0, total;
+#pragma unroll
+  for (int q = 0; q < kC; ++q) {
+    v[q] = count[kC * threadIdx.x + q];
+    sum += v[q];
+  }
+  int ex = block_exclusive_scan(sum, &total);   // its barriers separate the reads above from the writes below
+#pragma unroll
+  for (int q = 0; q < kC; ++q) {
+    const int c = kC * threadIdx.x + q;
+    count[c] = ex;
+    if (c <= nc) start[c] = ex;   // from nc on: n
+    ex += v[q];
+  }
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < kA; ++q) {
+    const int i = threadIdx.x + 1024 * q;
+    if (i < n) unsorted[count[cell[q]] + place[q]] = i;
+  }
 }
 
 // FP32 screen of the list build. Positions are held in units of the list radius from the grid's corner, one float4 per
@@ -252,11 +299,11 @@ __device__ __forceinline__ void list_end(int32_t i, int cnt, int maxnb, int32_t*
 // Neighbour lists, a warp per atom in cell order: the warp tests 32 candidates at a time by the FP32 screen and a ballot
 // keeps the accepted ones in stencil order, ascending index within a cell. WRAP: a periodic axis has fewer than 4
 // cells, so the image is found per pair instead of from the stencil offset (with 3 cells both images of a pair whose
-// images are in doubt lie outside the radius).
+// images are in doubt lie outside the radius). kU loads in flight.
 // Bound by instruction issue (about 30 per 32 candidates) and, in small systems, by the latency of one atom's chain. A
-// thread per atom testing every candidate in FP64 took, for the whole build, 305 us at 864 LJ atoms (now 42), 355 at
-// 16,384 (72) and 643 at 8000 ions with 250 neighbours (73).
-template <bool WRAP>
+// thread per atom testing every candidate in FP64 took, for the whole build, 305 us at 864 LJ atoms (now 23), 355 at
+// 16,384 (69) and 643 at 8000 ions with 250 neighbours (56).
+template <bool WRAP, int kU>
 __global__ void __launch_bounds__(kBlock) k_list_atoms(const double* __restrict__ pos, int64_t n,
                                                        const __grid_constant__ GridDev g, Screen f,
                                                        const int32_t* __restrict__ cell_of,
@@ -286,28 +333,37 @@ __global__ void __launch_bounds__(kBlock) k_list_atoms(const double* __restrict_
       my -= (float)((im / 3) % 3 - 1) * f.L[1];
       mz -= (float)(im / 9 - 1) * f.L[2];
     }
-    for (int base = s0; base < s1; base += 32) {
-      const int k = base + lane;
-      float4 o = make_float4(3e30f, 3e30f, 3e30f, 0.f);   // past the end: r^2 overflows, outside
-      if (k < s1) o = __ldg(screen + k);
-      float dx = o.x - mx, dy = o.y - my, dz = o.z - mz;
-      if (WRAP) {
-        dx -= f.L[0] * rintf(dx * f.inv[0]);
-        dy -= f.L[1] * rintf(dy * f.inv[1]);
-        dz -= f.L[2] * rintf(dz * f.inv[2]);
+    for (int base = s0; base < s1; base += 32 * kU) {
+      float4 o[kU];
+#pragma unroll
+      for (int v = 0; v < kU; ++v) {
+        const int k = base + 32 * v + lane;
+        o[v] = make_float4(3e30f, 3e30f, 3e30f, 0.f);   // past the end: r^2 overflows, outside
+        if (k < s1) o[v] = __ldg(screen + k);
       }
-      const float q = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
-      const int32_t j = __float_as_int(o.w);
-      bool in = k < s1 && q <= f.lo;
-      const bool band = k < s1 && !(q <= f.lo) && !(q >= f.hi);
-      if (__any_sync(0xffffffffu, band)) {
-        if (band) in = exact_pair(pos, i, j, g);
+#pragma unroll
+      for (int v = 0; v < kU; ++v) {
+        if (base + 32 * v >= s1) break;
+        const int k = base + 32 * v + lane;
+        float dx = o[v].x - mx, dy = o[v].y - my, dz = o[v].z - mz;
+        if (WRAP) {
+          dx -= f.L[0] * rintf(dx * f.inv[0]);
+          dy -= f.L[1] * rintf(dy * f.inv[1]);
+          dz -= f.L[2] * rintf(dz * f.inv[2]);
+        }
+        const float q = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
+        const int32_t j = __float_as_int(o[v].w);
+        bool in = k < s1 && q <= f.lo;
+        const bool band = k < s1 && !(q <= f.lo) && !(q >= f.hi);
+        if (__any_sync(0xffffffffu, band)) {
+          if (band) in = exact_pair(pos, i, j, g);
+        }
+        in = in && k != slot;
+        const unsigned bal = __ballot_sync(0xffffffffu, in);
+        const int at = cnt + __popc(bal & below);
+        if (in && at < maxnb) row[(int64_t)at * 32] = j;
+        cnt += __popc(bal);
       }
-      in = in && k != slot;
-      const unsigned bal = __ballot_sync(0xffffffffu, in);
-      const int at = cnt + __popc(bal & below);
-      if (in && at < maxnb) row[(int64_t)at * 32] = j;
-      cnt += __popc(bal);
     }
   }
   if (lane == 0) list_end(i, cnt, maxnb, nnb, status);
@@ -956,16 +1012,20 @@ int bin_cells(const double* pos, int64_t n, const acs_grid* g, void* work, cudaS
   int32_t* count = (int32_t*)w; w += align256((nc + 1) * 4);
   cb.start = (int32_t*)w; w += align256((nc + 1) * 4);
   int32_t* unsorted = (int32_t*)w; w += align256(n * 4);
+  int32_t* place = (int32_t*)w; w += align256(n * 4);
   int32_t* sums = (int32_t*)w;
   GridDev gd = to_dev(g);
-  if (cudaMemsetAsync(count, 0, (nc + 1) * 4, s) != cudaSuccess) return 1;
   const int nb = (int)ceil_div(n, kBlock);
-  k_bin<<<nb, kBlock, 0, s>>>(pos, n, gd, cb.cell_of, count);
-  k_scan_chunks<<<(int)nchunks, kScanThreads, 0, s>>>(count, cb.start, nc + 1, sums);
-  k_scan_sums<<<1, kScanThreads, 0, s>>>(sums, nchunks, nullptr);
-  k_scan_add<<<(int)nchunks, 256, 0, s>>>(cb.start, nc + 1, sums);
-  if (cudaMemsetAsync(count, 0, (nc + 1) * 4, s) != cudaSuccess) return 1;
-  k_scatter<<<nb, kBlock, 0, s>>>(cb.cell_of, n, cb.start, count, unsorted);
+  if (n <= kBinAtoms && nc < kBinCells) {
+    k_bin_block<<<1, 1024, 0, s>>>(pos, (int)n, gd, (int)nc, cb.cell_of, cb.start, unsorted);
+  } else {
+    if (cudaMemsetAsync(count, 0, (nc + 1) * 4, s) != cudaSuccess) return 1;
+    k_bin<<<nb, kBlock, 0, s>>>(pos, n, gd, cb.cell_of, place, count);
+    k_scan_chunks<<<(int)nchunks, kScanThreads, 0, s>>>(count, cb.start, nc + 1, sums);
+    k_scan_sums<<<1, kScanThreads, 0, s>>>(sums, nchunks, nullptr);
+    k_scan_add<<<(int)nchunks, 256, 0, s>>>(cb.start, nc + 1, sums);
+    k_scatter<<<nb, kBlock, 0, s>>>(cb.cell_of, place, n, cb.start, unsorted);
+  }
   k_rank_cells<<<nb, kBlock, 0, s>>>(pos, cb.cell_of, n, gd, screen_of(g, g->rc2), cb.start, unsorted, cb.screen);
   return 0;
 }
@@ -1035,7 +1095,7 @@ size_t acs_nlist_work_bytes(int64_t n, const acs_grid* g) {
   if (!g || n < 0) return 0;
   const int64_t nc = grid_cells(g);
   const int64_t nchunks = ceil_div(nc + 1, kScanChunk);
-  return 256 + align256((size_t)n * 16) + align256(n * 4) + 2 * align256((nc + 1) * 4) + align256(n * 4) +
+  return 256 + align256((size_t)n * 16) + align256(n * 4) + 2 * align256((nc + 1) * 4) + 2 * align256(n * 4) +
          align256((nchunks + 1) * 4);
 }
 
@@ -1060,7 +1120,12 @@ int acs_nlist_build(const double* pos, int64_t n, const acs_grid* g, int32_t max
     k_list_cells<<<dim3((unsigned)ceil_div(nc, kBlock / 32), chunks), kBlock, 0, s>>>(pos, gd, f, nc, cb.start, cb.screen,
                                                                                      maxnb, nbr, nnb, status);
   } else {
-    (wrap ? k_list_atoms<true> : k_list_atoms<false>)<<<(int)ceil_div(n, kBlock / 32), kBlock, 0, s>>>(
+    // 4 loads in flight where a stretch of 3 cells fills them (4096 ions in 27 cells: 53 us with 1, 49 with 2, 45 with 4),
+    // else 2 (8000 ions in 216 cells: 41, 36, 39)
+    const bool long_rows = 3 * n >= 256 * nc;
+    auto kernel = wrap ? (long_rows ? k_list_atoms<true, 4> : k_list_atoms<true, 2>)
+                       : (long_rows ? k_list_atoms<false, 4> : k_list_atoms<false, 2>);
+    kernel<<<(int)ceil_div(n, kBlock / 32), kBlock, 0, s>>>(
         pos, n, gd, f, cb.cell_of, cb.start, cb.screen, maxnb, nbr, nnb, status);
   }
   return launch_status();

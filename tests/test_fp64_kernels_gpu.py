@@ -85,7 +85,7 @@ def _reference_lists(pos, g):
 
 # (cells per axis, atoms, periodic): one cell, the image found per pair (3 cells), stencil images (4 and more), a warp
 # per cell (1024 cells and more) with ragged and with crowded cells, open boxes
-LIST_FORMS = [((1, 1, 1), 70, True), ((3, 3, 3), 500, True), ((4, 3, 7), 900, True), ((4, 4, 5), 33, True),
+LIST_FORMS = [((1, 1, 1), 70, True), ((3, 3, 3), 2700, True), ((3, 3, 3), 500, True), ((4, 3, 7), 900, True), ((4, 4, 5), 33, True),
               ((5, 4, 6), 1300, True), ((11, 10, 10), 4500, True), ((4, 16, 17), 4400, True), ((12, 11, 9), 4800, False),
               ((2, 2, 3), 400, False)]
 
@@ -498,3 +498,30 @@ def test_training_step_gradient(n):
         assert np.array_equal(a, b)
     assert np.linalg.norm(out[0][0] - ref) <= 3e-2 * np.linalg.norm(ref)
     assert abs(out[0][2].sum() - loss.item()) <= 1e-2 * loss.item()
+
+
+# the one-block binning's limits: 8192 atoms, 8191 cells, one over each
+@pytest.mark.parametrize("n,cells", [(8192, (10, 10, 10)), (8193, (10, 10, 10)), (5000, (21, 13, 30)), (5000, (21, 15, 26)),
+                                     (5000, (16, 16, 32))])
+def test_list_binning_limits(n, cells):
+    """Neighbour counts by brute force at the sizes where the binning changes; entries ascend within a cell, so the two
+    binnings agree entry by entry with the reference lists of a sample of atoms. Exact."""
+    torch, L, st = _abi()
+    rng = np.random.default_rng(n)
+    rc = 1.0
+    box = (np.array(cells) + 0.3) * rc
+    pos = rng.uniform(0, 1, (n, 3)) * box
+    g = _grid(L, box, rc)
+    assert tuple(g.ncell) == cells
+    p, b = torch.from_numpy(pos).cuda(), torch.from_numpy(box).cuda()
+    nbr, nnb = _build_list(torch, L, st, p, g, 64)
+    d = p[None, :, :] - p[:1000, None, :]
+    d = d - b * torch.round(d / b)
+    close = (d[..., 0] * d[..., 0] + d[..., 1] * d[..., 1]) + d[..., 2] * d[..., 2] < rc ** 2
+    assert torch.equal(nnb[:1000].long(), close.sum(1) - 1)
+    rows = nbr.view(-1, 64, 32)
+    for i in range(0, 1000, 37):
+        got = rows[i // 32, : int(nnb[i]), i % 32].cpu().numpy()
+        cell = np.minimum((pos / box * cells).astype(int), np.array(cells) - 1)
+        rank = ((cell[got] - cell[i] + 1) % cells) @ np.array([9, 3, 1])
+        assert np.array_equal(got, got[np.lexsort((got, rank))])
