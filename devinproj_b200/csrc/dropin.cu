@@ -619,14 +619,34 @@ __global__ void k_pairs(const int32_t* __restrict__ nbr, const int32_t* __restri
   }
 }
 
-__global__ void k_displacement(const double* __restrict__ pos, const double* __restrict__ pos0, int64_t n, ImageBox box,
-                               double half_skin2, int32_t* flag) {
-  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
+__device__ __forceinline__ bool moved(const double* __restrict__ pos, const double* __restrict__ pos0, int64_t i,
+                                      const ImageBox& box, double half_skin2) {
   double dx = sub(pos[3 * i], pos0[3 * i]), dy = sub(pos[3 * i + 1], pos0[3 * i + 1]),
          dz = sub(pos[3 * i + 2], pos0[3 * i + 2]);
   image3(dx, dy, dz, box);
-  if (!(norm2(dx, dy, dz) < half_skin2)) *flag = 1;  // NaN also forces a rebuild, as in the reference
+  return !(norm2(dx, dy, dz) < half_skin2);   // NaN also forces a rebuild, as in the reference
+}
+
+// One block's answer for up to kMovedAtoms atoms, without the clear that the grid's needs before it: a small system's
+// skin test is launches (a clear and a kernel, 3 us, for 2 us of one kernel).
+constexpr int kMovedAtoms = 4096;
+__global__ void __launch_bounds__(1024) k_displacement_block(const double* __restrict__ pos,
+                                                             const double* __restrict__ pos0, int n, ImageBox box,
+                                                             double half_skin2, int32_t* flag) {
+  bool any = false;
+#pragma unroll
+  for (int q = 0; q < kMovedAtoms / 1024; ++q) {
+    const int i = threadIdx.x + 1024 * q;
+    if (i < n) any = any || moved(pos, pos0, i, box, half_skin2);
+  }
+  const int r = __syncthreads_or(any);
+  if (threadIdx.x == 0) *flag = r ? 1 : 0;
+}
+
+__global__ void k_displacement(const double* __restrict__ pos, const double* __restrict__ pos0, int64_t n, ImageBox box,
+                               double half_skin2, int32_t* flag) {
+  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n && moved(pos, pos0, i, box, half_skin2)) *flag = 1;
 }
 
 // ------------------------------------------------------------------------------------ forces --
@@ -922,15 +942,30 @@ __device__ __forceinline__ double py_mod(double x, double L) {
   return r;
 }
 
-__global__ void k_drift_wrap(double* __restrict__ pos, const double* __restrict__ vel, int64_t n, double dt, ImageBox box) {
-  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
+// Calls f(element, atom, axis) for the 768 components of each block's 256 atoms, three per thread, 256 apart: the arrays
+// stream, where an atom per thread reads and writes 24-byte strides.
+template <class F>
+__device__ __forceinline__ void for_components(int64_t n, F&& f) {
+  const int64_t i0 = (int64_t)blockIdx.x * kBlock;
+  const int m = (int)min((int64_t)kBlock, n - i0) * 3;
 #pragma unroll
-  for (int d = 0; d < 3; ++d) {
-    double x = add(pos[3 * i + d], mul(dt, vel[3 * i + d]));
-    if (box.periodic) x = py_mod(x, box.L[d]);
-    pos[3 * i + d] = x;
+  for (int q = 0; q < 3; ++q) {
+    const int l = threadIdx.x + kBlock * q;
+    if (l < m) f(3 * i0 + l, i0 + l / 3, l % 3);
   }
+}
+
+// pos += dt vel, pos %= L. In (0, L) the remainder is x itself, in (L, 2L) and (-L, 0) one exact or IEEE subtraction or
+// addition, as py_mod's fmod has it; its loop is left to the others. 1M atoms 22 -> 12 us (its bytes take 11.5).
+__global__ void k_drift_wrap(double* __restrict__ pos, const double* __restrict__ vel, int64_t n, double dt, ImageBox box) {
+  for_components(n, [&](int64_t e, int64_t, int d) {
+    double x = add(pos[e], mul(dt, vel[e]));
+    if (box.periodic) {
+      const double L = d == 0 ? box.L[0] : d == 1 ? box.L[1] : box.L[2];
+      if (!(x > 0.0 && x < L)) x = x > L && x < 2.0 * L ? sub(x, L) : (x < 0.0 && x > -L ? add(x, L) : py_mod(x, L));
+    }
+    pos[e] = x;
+  });
 }
 
 // Langevin O-step: vel = c1 * vel + sig[atom] * noise (accusim/integrators.py:66-67, no FMA).
@@ -945,12 +980,8 @@ struct MassTab {
 };
 
 __global__ void k_accel(double* __restrict__ acc, const double* __restrict__ force, const int32_t* __restrict__ sp,
-                        MassTab mt, int64_t n) {
-  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const double m = mt.m[sp[i]];
-#pragma unroll
-  for (int d = 0; d < 3; ++d) acc[3 * i + d] = div(force[3 * i + d], m);
+                        const __grid_constant__ MassTab mt, int64_t n) {
+  for_components(n, [&](int64_t e, int64_t i, int) { acc[e] = div(force[e], mt.m[sp[i]]); });   // 1M atoms 20 -> 11 us
 }
 
 __global__ void __launch_bounds__(kBlock) k_conserved(const double* __restrict__ pos, const double* __restrict__ vel,
@@ -1168,10 +1199,14 @@ int acs_nlist_displacement(const double* pos, const double* pos0, int64_t n, con
                            double half_skin2, int32_t* flag_dev, void* stream) {
   if (n < 0 || !flag_dev || (n > 0 && (!pos || !pos0))) return ACS_ERR_ARG;
   cudaStream_t s = (cudaStream_t)stream;
+  const ImageBox box = image_box(box3, periodic);
+  if (n > 0 && n <= kMovedAtoms) {
+    k_displacement_block<<<1, 1024, 0, s>>>(pos, pos0, (int)n, box, half_skin2, flag_dev);
+    return launch_status();
+  }
   if (cudaMemsetAsync(flag_dev, 0, 4, s) != cudaSuccess) return ACS_ERR_CUDA;
   if (n == 0) return ACS_OK;
-  k_displacement<<<(int)ceil_div(n, kBlock), kBlock, 0, s>>>(pos, pos0, n, image_box(box3, periodic), half_skin2,
-                                                              flag_dev);
+  k_displacement<<<(int)ceil_div(n, kBlock), kBlock, 0, s>>>(pos, pos0, n, box, half_skin2, flag_dev);
   return launch_status();
 }
 

@@ -525,3 +525,47 @@ def test_list_binning_limits(n, cells):
         cell = np.minimum((pos / box * cells).astype(int), np.array(cells) - 1)
         rank = ((cell[got] - cell[i] + 1) % cells) @ np.array([9, 3, 1])
         assert np.array_equal(got, got[np.lexsort((got, rank))])
+
+
+@pytest.mark.parametrize("n", [1, 85, 256, 257, 1000, 4096, 4097, 70001])
+def test_integrator_kernels(n):
+    """Drift and wrap, acceleration and the skin test against NumPy, bit for bit: coordinates inside the box, on its edges,
+    one and several boxes away, signed zeros, not finite; the moved atom first, last and absent."""
+    torch, L, st = _abi()
+    rng = np.random.default_rng(n)
+    box = np.array([2.0, 3.7, 1.3])
+    pos = rng.uniform(-0.3, 1.3, (n, 3)) * box
+    vel = rng.normal(0, 0.2, (n, 3))
+    special = np.array([0.0, -0.0, 1.0, -1.0, 2.0, -2.0, 5.5, -7.25, 1e9, np.nan, np.inf, -np.inf, 1e-320, -1e-320])
+    k = min(n, 14)
+    pos[:k], vel[:k] = (special[:k, None] * box), 0.0
+    dt = 0.37
+    with np.errstate(invalid="ignore"):
+        ref = np.remainder(pos + dt * vel, box)
+    p, v = torch.from_numpy(pos).cuda(), torch.from_numpy(vel).cuda()
+    assert L.acs_vv_drift_wrap(p.data_ptr(), v.data_ptr(), n, dt, box.ctypes.data, 1, st) == 0
+    got = p.cpu().numpy()
+    assert np.array_equal(got, ref, equal_nan=True) and np.array_equal(np.signbit(got[~np.isnan(ref)]), np.signbit(ref[~np.isnan(ref)]))
+    sp = rng.integers(0, 3, n).astype(np.int32)
+    m = np.array([1.7, 22.99, 39.948])
+    s, acc = torch.from_numpy(sp).cuda(), torch.empty_like(v)
+    assert L.acs_vv_accel(acc.data_ptr(), v.data_ptr(), s.data_ptr(), m.ctypes.data, 3, n, st) == 0
+    assert np.array_equal(acc.cpu().numpy(), vel / m[sp][:, None])
+    a = rng.uniform(0, 1, (n, 3)) * box
+    b = (a + rng.uniform(-0.05, 0.05, (n, 3))) % box
+    b[:1] = (a[:1] + [0.2, 0.0, 0.0]) % box
+    flag = torch.full((1,), 7, dtype=torch.int32, device="cuda")
+    ad = torch.from_numpy(a).cuda()
+    for where in (0, n - 1, None):
+        c = b.copy()
+        if where != 0:
+            c[0] = a[0]
+        if where:
+            c[where] = (a[where] + [0.0, 0.2, 0.0]) % box
+        cd = torch.from_numpy(c).cuda()
+        assert L.acs_nlist_displacement(cd.data_ptr(), ad.data_ptr(), n, box.ctypes.data, 1, 0.15 ** 2, flag.data_ptr(), st) == 0
+        assert int(flag.item()) == (0 if where is None else 1)
+    c[n // 2] = np.nan
+    cd = torch.from_numpy(c).cuda()
+    assert L.acs_nlist_displacement(cd.data_ptr(), ad.data_ptr(), n, box.ctypes.data, 1, 0.15 ** 2, flag.data_ptr(), st) == 0
+    assert int(flag.item()) == 1
