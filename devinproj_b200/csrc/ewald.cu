@@ -98,23 +98,30 @@ __device__ __forceinline__ double2 cmul(double2 a, double2 b) {
 }
 __device__ __forceinline__ double2 conj_if(double2 a, bool neg) { return make_double2(a.x, neg ? -a.y : a.y); }
 
-// partial[c][k] = sum_{j in chunk c} q_j (cos, sin)(k . r_j)     (accusim/forces.py:382-383). A thread per k-vector; the
-// chunk's tables pass through shared memory, where consecutive vectors (the last axis fastest) read consecutive
-// entries. With the tables 10 FP64 operations per atom and pair of mirrored vectors, without some 60 per vector.
+// partial[c][k] = sum_{j in chunk c} q_j (cos, sin)(k . r_j)     (accusim/forces.py:382-383). A thread per k-vector, 32
+// atoms at a time. The block's vectors share few pairs of the first two coordinates (runs along the last axis): the
+// products q e^{ikx x} e^{iky y} of up to kRuns runs are formed once per atom in shared memory, and a vector adds the
+// four real products with e^{ikz z}, 4 FP64 operations and two reads per atom and pair of mirrored vectors (three
+// factors per vector, 10 operations and three reads: 69 us at 8000 ions and 7152 vectors, 50 here; a sine and cosine
+// per atom and vector 226). More runs than that in a block form the three factors per vector.
+constexpr int kRuns = 32;
 __global__ void __launch_bounds__(kBlock) k_sfac_partial(const Packed* __restrict__ pk, int64_t n,
                                                          const double* __restrict__ kv, const int32_t* __restrict__ kn,
                                                          const double* __restrict__ wfold, int K,
                                                          const double2* __restrict__ table,
                                                          const KForm* __restrict__ form, double2* __restrict__ partial) {
-  __shared__ double2 tab[kAtoms][3 * kTab];
-  __shared__ double charge[kAtoms];
+  __shared__ double2 ez[kAtoms][kTab];
+  __shared__ double2 exy[kAtoms][kRuns];
+  __shared__ int codes[kRuns];
+  __shared__ int before[kWarps];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   const int c = blockIdx.y;
   const int64_t per = (n + kSChunks - 1) / kSChunks;
   const int64_t j0 = c * per, j1 = min(n, j0 + per);
-  double re = 0.0, im = 0.0;
   if (form->general) {
     if (k >= K) return;
+    double re = 0.0, im = 0.0;
     const double kx = kv[3 * k], ky = kv[3 * k + 1], kz = kv[3 * k + 2];
     for (int64_t j = j0; j < j1; ++j) {
       const Packed o = ld_packed(pk + j);
@@ -127,25 +134,58 @@ __global__ void __launch_bounds__(kBlock) k_sfac_partial(const Packed* __restric
     return;
   }
   const bool on = k < K && wfold[k] != 0.0;
+  if (!__syncthreads_or(on)) return;   // a block of the mirrored half
   const int code = k < K ? kn[k] : 0x101010;
   const int x = (code & 255) - 16, y = (code >> 8 & 255) - 16, z = (code >> 16 & 255) - 16;
-  const int ax = abs(x), ay = kTab + abs(y), az = 2 * kTab + abs(z);
-  if (!__syncthreads_or(on)) return;   // a block of the mirrored half
+  // the runs of equal (x, y) among the block's vectors, numbered in order
+  const bool first = on && (threadIdx.x == 0 || wfold[k - 1] == 0.0 || (kn[k - 1] & 0xffff) != (code & 0xffff));
+  const unsigned bal = __ballot_sync(0xffffffffu, first);
+  if (lane == 0) before[warp] = __popc(bal);
+  __syncthreads();
+  int run = __popc(bal & (0xffffffffu >> (31 - lane))) - 1, runs = 0;
+  for (int w = 0; w < kWarps; ++w) {
+    if (w < warp) run += before[w];
+    runs += before[w];
+  }
+  const bool few = runs <= kRuns;
+  if (few && first) codes[run] = code & 0xffff;
+  double cc = 0.0, ss = 0.0, cs = 0.0, sc = 0.0;   // sums of the products of (re, im) of exy with (cos, sin) of ez
   for (int64_t b = j0; b < j1; b += kAtoms) {
     const int m = (int)min((int64_t)kAtoms, j1 - b);
     __syncthreads();
-    for (int t = threadIdx.x; t < m * 3 * kTab; t += blockDim.x) tab[t / (3 * kTab)][t % (3 * kTab)] = table[b * 3 * kTab + t];
-    if ((int)threadIdx.x < m) charge[threadIdx.x] = pk[b + threadIdx.x].w;
+    for (int t = threadIdx.x; t < m * kTab; t += blockDim.x)
+      ez[t / kTab][t % kTab] = table[(b + t / kTab) * 3 * kTab + 2 * kTab + t % kTab];
+    if (few) {
+      for (int t = threadIdx.x; t < m * runs; t += blockDim.x) {
+        const int j = t / runs, r = t % runs, rx = (codes[r] & 255) - 16, ry = (codes[r] >> 8) - 16;
+        const double2* tj = table + (b + j) * 3 * kTab;
+        const double2 e = cmul(conj_if(tj[abs(rx)], rx < 0), conj_if(tj[kTab + abs(ry)], ry < 0));
+        const double q = pk[b + j].w;
+        exy[j][r] = make_double2(q * e.x, q * e.y);
+      }
+    }
     __syncthreads();
     if (on) {
-      for (int j = 0; j < m; ++j) {   // x >= 0 in the half that is summed
-        const double2 e = cmul(cmul(tab[j][ax], conj_if(tab[j][ay], y < 0)), conj_if(tab[j][az], z < 0));
-        re = fma(charge[j], e.x, re);
-        im = fma(charge[j], e.y, im);
+      for (int j = 0; j < m; ++j) {
+        double2 p;
+        if (few) {
+          p = exy[j][run];
+        } else {
+          const double2* tj = table + (b + j) * 3 * kTab;
+          p = cmul(conj_if(tj[abs(x)], x < 0), conj_if(tj[kTab + abs(y)], y < 0));
+          const double q = pk[b + j].w;
+          p.x *= q;
+          p.y *= q;
+        }
+        const double2 e = ez[j][abs(z)];
+        cc = fma(p.x, e.x, cc);
+        ss = fma(p.y, e.y, ss);
+        cs = fma(p.x, e.y, cs);
+        sc = fma(p.y, e.x, sc);
       }
     }
   }
-  if (on) partial[(int64_t)c * K + k] = make_double2(re, im);
+  if (on) partial[(int64_t)c * K + k] = z < 0 ? make_double2(cc + ss, sc - cs) : make_double2(cc - ss, sc + cs);
 }
 
 // S'_k = w_k S_k (a pair's weight on the half that stands for both) and sum_k w |S|^2.
@@ -186,8 +226,9 @@ __device__ __forceinline__ double ewald_pair(const EwaldPar& P, double r2, doubl
 // through the lanes: 32 rounds of 32 different pairs, after which the forces on the tile are home; those of the block's
 // warps are added in warp order and stored per block, so every sum has a fixed order. Its own tile a warp takes both
 // ways round. Bound by FP64 issue, some 95 operations per round whether few or all of its pairs are inside rcut; the
-// rotation (14 shuffles) hides behind them. 8000 ions: 0.29 ms; the pairs from both sides, a lane per atom (k_ewald_real),
-// 0.55; the whole sum went from 9.75 ms (one thread per atom for all pairs and vectors) to 0.46.
+// rotation (14 shuffles) hides behind them. 8000 ions: 0.27 ms in 112 parts of a block row (0.29 in 56, 0.34 in 28: a
+// block's share of the triangle shrinks along the rows); the pairs from both sides, a lane per atom (k_ewald_real),
+// 0.55; the whole sum went from 9.75 ms (one thread per atom for all pairs and vectors) to 0.42.
 __global__ void __launch_bounds__(kBlock, 3) k_ewald_tiles(const Packed* __restrict__ pk, int64_t n,
                                                            const __grid_constant__ EwaldPar P,
                                                            Packed* __restrict__ ipart, double* __restrict__ jpart) {
@@ -442,7 +483,7 @@ int split_of(int64_t rows, int64_t rounds, int64_t most) {
   return (int)std::max<int64_t>(1, std::min<int64_t>(most, ceil_div(444 * rounds, std::max<int64_t>(rows, 1))));
 }
 int real_chunks(int64_t n) {
-  return n <= kTileAtoms ? split_of(ceil_div(n, kBlock), 4, std::min<int64_t>(64, ceil_div(n, 32)))
+  return n <= kTileAtoms ? split_of(ceil_div(n, kBlock), 8, std::min<int64_t>(128, ceil_div(n, 32)))
                          : split_of(ceil_div(n, kAtoms), 4, 64);
 }
 int recip_shares(int64_t n) { return split_of(ceil_div(n, kAtoms), 3, 16); }
