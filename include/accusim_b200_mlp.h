@@ -18,8 +18,11 @@
 extern "C" {
 #endif
 
+/* About 5 KB per atom up to 49,152 atoms (phase factors, real-space parts), 3 KB above, and 1 KB per k-vector. */
 size_t acs_ewald_work_bytes(int64_t n, int32_t K);
 /* pos (n x 3, m), q (n, C), kvec (K x 3, 1/m) and kw (K) are device arrays. force = k * f (N);
+ * Any k-vectors are taken; a set of small integer multiples of 2 pi / box edge that holds each vector's mirror image
+ * once (the reference's) runs on tabulated phase factors, decided on the device at each call.
  * energy3_dev[0] = real-space pair sum (unscaled), [1] = sum_k w_k |S_k|^2 (unscaled): the host forms
  * U = k * (energy3[0] + 2 pi / V * energy3[1] - alpha / sqrt(pi) * sum q^2). */
 int acs_ewald_fp64(const double* pos, const double* q, int64_t n, const double* box3, const double* kvec,
