@@ -684,12 +684,23 @@ struct PairSplit {
   int64_t blocks;
 };
 
-// Enough threads for the chip: the fewest phases that give kPairThreads, at most 32.
-constexpr int64_t kPairThreads = 131072;
-PairSplit pair_split(int64_t n) {
+// The fewest phases (at most 32) that give `threads`, then more while each thread keeps kPhaseEntries of the `entries`
+// an atom has room for, up to kMostThreads in all. 151,552 threads are resident, so a split below that leaves places
+// empty, one of a few waves loses its last one, and a thread with few entries is all prologue. DSF terms are long enough
+// to want several waves: 32,768 ions 141 us at 131,072 threads, 118 at 262,144, 112 at 524,288; 175,616 ions 678, 595,
+// 544; 64,000 ions 224, 213, 205 (209 at 1,048,576). LJ with 79 entries an atom does not: 32,000 atoms 18.5 us at
+// 128,000 threads, 21.6 at 256,000, 21.5 at 64,000; 55,296 atoms 25.5 at 110,592, 28.0 at 221,184, 35.0 at 55,296;
+// 1,048,576 atoms 0.355 ms with one phase, 0.372 with two, 0.430 with four. With 351 entries it does: 110,592 ions
+// 135 us with four phases, 157 with two, 147 with eight; 175,616 ions 210 with four, 300 with one.
+constexpr int64_t kMostThreads = 1 << 20, kLjThreads = 98304, kDsfThreads = 524288;
+constexpr int kPhaseEntries = 80;
+PairSplit pair_split(int64_t n, int64_t threads, int64_t entries) {
   PairSplit s;
   s.log2_phases = 0;
-  while (s.log2_phases < 5 && (n << s.log2_phases) < kPairThreads) ++s.log2_phases;
+  while (s.log2_phases < 5 && (n << s.log2_phases) < threads) ++s.log2_phases;
+  while (s.log2_phases < 5 && (n << (s.log2_phases + 1)) <= kMostThreads &&
+         entries >> (s.log2_phases + 1) >= kPhaseEntries)
+    ++s.log2_phases;
   s.atoms = kBlock >> s.log2_phases;
   s.blocks = ceil_div(n, s.atoms);
   return s;
@@ -842,7 +853,7 @@ template <bool PACKED, bool ONE>
 void launch_lj64(const double* pos, const int32_t* sp, const Packed* pk, int64_t n, const ImageBox& b, const int32_t* nbr,
                  const int32_t* nnb, int maxnb, const LJTab& t, double* force, double* partials, unsigned int* ticket,
                  double* energy, cudaStream_t s) {
-  const PairSplit split = pair_split(n);
+  const PairSplit split = pair_split(n, kLjThreads, nbr ? maxnb : n);
   if (nbr)
     k_lj64<false, PACKED, ONE><<<(int)split.blocks, kBlock, 0, s>>>(pos, sp, pk, n, b, nbr, nnb, maxnb, t, split, force,
                                                                     partials, ticket, energy);
@@ -1212,7 +1223,10 @@ int acs_nlist_displacement(const double* pos, const double* pos0, int64_t n, con
 
 // Energy partials (one per block of the pair kernels), ticket, packed positions; 256 bytes to align them in the
 // caller's buffer.
-static int64_t force_blocks(int64_t n) { return pair_split(std::max<int64_t>(n, 1)).blocks; }
+static int64_t force_blocks(int64_t n) {   // the most of any split: more than one phase ends at kMostThreads
+  n = std::max<int64_t>(n, 1);
+  return std::max(ceil_div(n, kBlock), std::min<int64_t>(ceil_div(n, kBlock / 32), kMostThreads / kBlock));
+}
 size_t acs_force_work_bytes(int64_t n) {
   return align256(force_blocks(n) * 8) + 256 + align256((size_t)std::max<int64_t>(n, 1) * sizeof(Packed)) + 256;
 }
@@ -1283,7 +1297,7 @@ int acs_dsf_fp64(const double* pos, const double* q, int64_t n, const double* bo
   P.fshift = P.erc / (rcut * rcut) + P.c * exp(-((alpha * rcut) * (alpha * rcut))) / rcut;
   P.self_coef = P.erc / (2.0 * rcut) + alpha / sqrt(M_PI);
   const ImageBox b = image_box(box3, periodic);
-  const PairSplit split = pair_split(n);
+  const PairSplit split = pair_split(n, kDsfThreads, 0);
   if (nbr)
     k_dsf64<false><<<(int)split.blocks, kBlock, 0, s>>>(pk, n, b, nbr, nnb, maxnb, ex_start, ex_idx, P, split, force,
                                                        partials, ticket, energy_dev);

@@ -174,7 +174,7 @@ def _scatter(n, i, x):
     return np.stack([np.bincount(i, x[:, k], minlength=n) for k in range(3)], 1)
 
 
-# atoms: the pair kernels' splits change at 8, 4096 (32 -> 16 phases at 131,072 threads), 8192; blocks end ragged
+# atoms: a block holds 8 (32 phases) or 16 (n = 8193); blocks end ragged
 @pytest.mark.parametrize("n", [1, 2, 7, 9, 255, 257, 399, 4095, 4097, 8193])
 @pytest.mark.parametrize("species", [1, 3])
 @pytest.mark.parametrize("periodic", [True, False])
@@ -289,6 +289,59 @@ def test_dsf_forces(n, dense, alpha):
     tol = (260 + 4 * (alpha * rc) ** 2) * EPS
     assert np.all(np.abs(force.cpu().numpy() - F) <= tol * mag + 1e-300)
     assert abs(energy.item() - U) <= tol * Umag
+
+
+# copies of 512 atoms: 13,824 (LJ 8 phases, DSF 32), 32,768 (4, 16), 110,592 (4, 8), 262,144 (4, 2), 626,688 (1, 1)
+@pytest.mark.parametrize("copies", [(3, 3, 3), (4, 4, 4), (6, 6, 6), (8, 8, 8), (8, 9, 17)])
+def test_pair_splits(copies):
+    """Every copy of a periodic system feels the system's own forces. A copy's coordinates are rounded at the whole box's
+    size, L eps / 2 each, so a pair's distance is off by at most 2 sqrt(3) L eps and its term by 16 times that over the
+    smallest distance (LJ's steepest power 14, DSF's less); to that the bounds of the direct comparisons."""
+    from scipy.special import erfc
+    torch, L, st = _abi()
+    rng = np.random.default_rng(11)
+    rc, alpha, kc = 2.5, 0.8, 1.7
+    box = np.array([8.6, 8.8, 8.5])
+    grid = np.stack(np.meshgrid(*[np.arange(8)] * 3, indexing="ij"), -1).reshape(-1, 3)
+    pos = (grid + 0.5 + rng.normal(0, 0.06, (512, 3))) * box / 8
+    q = np.where(np.arange(512) % 2 == 0, 1.0, -1.2)
+    i, j, d, r2 = _pairs_within(pos, box, rc)
+    s6, c6, r = r2 ** -3.0, rc ** -6.0, np.sqrt(r2)
+    c, erc, qq = 2 * alpha / np.sqrt(np.pi), erfc(alpha * rc), q[i] * q[j]
+    sh = erc / rc ** 2 + c * np.exp(-(alpha * rc) ** 2) / rc
+    g = erfc(alpha * r) / r ** 2 + c * np.exp(-(alpha * r) ** 2) / r
+    er, self_u = erfc(alpha * r) / r, np.sum(q ** 2) * (erc / (2 * rc) + alpha / np.sqrt(np.pi))
+    want = [(_scatter(512, i, (-24 * (2 * s6 ** 2 - s6) / r2)[:, None] * d),
+             _scatter(512, i, (24 * (2 * s6 ** 2 + s6) / r2)[:, None] * np.abs(d)),
+             0.5 * np.sum(4 * (s6 ** 2 - s6 - (c6 ** 2 - c6))), 0.5 * np.sum(4 * (s6 ** 2 + s6 + 1))),
+            (kc * _scatter(512, i, -(qq * (g - sh) / r)[:, None] * d),
+             kc * _scatter(512, i, (np.abs(qq) * (g + sh) / r)[:, None] * np.abs(d)),
+             kc * (0.5 * np.sum(qq * (er - erc / rc + sh * (r - rc))) - self_u),
+             kc * (0.5 * np.sum(np.abs(qq) * (er + erc / rc + sh * (rc - r))) + self_u))]
+    shift = np.stack(np.meshgrid(*[np.arange(k) for k in copies], indexing="ij"), -1).reshape(-1, 1, 3) * box
+    whole = box * copies
+    many, times = (pos + shift).reshape(-1, 3), int(np.prod(copies))
+    n = len(many)
+    p, qd = torch.from_numpy(many).cuda(), torch.from_numpy(np.tile(q, times)).cuda()
+    sp = torch.zeros(n, dtype=torch.int32, device="cuda")
+    maxnb = 400 if n < 300000 else 128
+    nbr, nnb = _build_list(torch, L, st, p, _grid(L, whole, rc + 0.3), maxnb)
+    one, b = np.ones((1, 1)), np.ascontiguousarray(whole)
+    tol = (400 + 4 * (alpha * rc) ** 2 + 16 * 2 * 3 ** 0.5 * whole.max() / r.min()) * EPS
+    for kind, (F, mag, U, Umag) in zip(("lj", "dsf"), want):
+        force = torch.full((n, 3), float("nan"), dtype=torch.float64, device="cuda")
+        energy = torch.full((1,), float("nan"), dtype=torch.float64, device="cuda")
+        work = torch.empty(L.acs_force_work_bytes(n), dtype=torch.uint8, device="cuda")
+        tail = (force.data_ptr(), energy.data_ptr(), work.data_ptr(), work.numel(), st)
+        if kind == "lj":
+            assert L.acs_lj_fp64(p.data_ptr(), sp.data_ptr(), n, b.ctypes.data, 1, nbr.data_ptr(), nnb.data_ptr(), maxnb, 1,
+                                 one.ctypes.data, one.ctypes.data, rc, *tail) == 0
+        else:
+            assert L.acs_dsf_fp64(p.data_ptr(), qd.data_ptr(), n, b.ctypes.data, 1, nbr.data_ptr(), nnb.data_ptr(), maxnb,
+                                  None, None, alpha, rc, kc, *tail) == 0
+        got = force.cpu().numpy().reshape(times, 512, 3)
+        assert np.all(np.abs(got - F) <= tol * mag)
+        assert abs(energy.item() / times - U) <= tol * Umag
 
 
 def _ewald_vectors(kind, box, alpha):
