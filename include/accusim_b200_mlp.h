@@ -18,7 +18,7 @@
 extern "C" {
 #endif
 
-/* About 5 KB per atom up to 49,152 atoms (phase factors, real-space parts), 3 KB above, and 1 KB per k-vector. */
+/* 2.5 to 6.1 KB per atom up to 49,152 atoms (phase factors, real-space parts), 1 KB above, and 1 KB per k-vector. */
 size_t acs_ewald_work_bytes(int64_t n, int32_t K);
 /* pos (n x 3, m), q (n, C), kvec (K x 3, 1/m) and kw (K) are device arrays. force = k * f (N);
  * Any k-vectors are taken; a set of small integer multiples of 2 pi / box edge that holds each vector's mirror image
