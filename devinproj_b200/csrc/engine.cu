@@ -919,8 +919,11 @@ __device__ __noinline__ bool band_accept(const double* __restrict__ xa, int64_t 
 template <bool EX, bool ATOMS>
 __global__ void __launch_bounds__(256, ATOMS ? 2 : 3) k_rebuild(Eng E, int dst, int rec, int rec_idx, int force_all) {
   __shared__ unsigned char fl[kMaxRep];
-  __shared__ int any_s;
-  if (threadIdx.x == 0) any_s = 0;
+  __shared__ int any_s, err_s;
+  if (threadIdx.x == 0) {
+    any_s = 0;
+    err_s = E.status->flags & (ACS_FLAG_OVERFLOW | ACS_FLAG_NONFINITE | ACS_FLAG_TIMEOUT);
+  }
   __syncthreads();
   int local_any = 0;
   for (int r = threadIdx.x; r < E.R; r += blockDim.x) {
@@ -931,7 +934,9 @@ __global__ void __launch_bounds__(256, ATOMS ? 2 : 3) k_rebuild(Eng E, int dst, 
   if (local_any) atomicOr(&any_s, 1);
   __syncthreads();
   const bool any = any_s != 0;
-  const bool err0 = (E.status->flags & (ACS_FLAG_OVERFLOW | ACS_FLAG_NONFINITE | ACS_FLAG_TIMEOUT)) != 0;
+  // Whether the kernel runs at all has to be the same answer in every thread of the grid: one read per block, and no
+  // block sets a flag before a grid barrier has shown that all of them have read it.
+  const bool err0 = err_s != 0;
   const int64_t gtid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int64_t gstride = (int64_t)gridDim.x * blockDim.x;
 
@@ -1021,6 +1026,7 @@ __global__ void __launch_bounds__(256, ATOMS ? 2 : 3) k_rebuild(Eng E, int dst, 
   }
   PHASE(1);
   // P1: absolute wrapped positions, new cells, arrival number within the cell
+  bool bad = false;   // a position that is not finite: reported after the barrier
   for_flagged_slots(E, gtid, gstride, [&](int64_t s, int r) {
     const RepDev& R = E.rep[r];
     int c0, c1, c2;
@@ -1039,7 +1045,7 @@ __global__ void __launch_bounds__(256, ATOMS ? 2 : 3) k_rebuild(Eng E, int dst, 
       E.xa[3 * s + d] = x[d];
     }
     if (!fin) {
-      atomicOr(&E.status->flags, ACS_FLAG_NONFINITE);
+      bad = true;
       nc3[0] = nc3[1] = nc3[2] = 0;
     }
     const int c = R.cellbase + (nc3[0] * R.nc[1] + nc3[1]) * R.nc[2] + nc3[2];
@@ -1047,6 +1053,7 @@ __global__ void __launch_bounds__(256, ATOMS ? 2 : 3) k_rebuild(Eng E, int dst, 
     E.place[s] = atomicAdd(&E.count[c], 1);
   });
   if (!grid_sync(E.bar, E.status, E.spin_limit)) return;
+  if (bad) atomicOr(&E.status->flags, ACS_FLAG_NONFINITE);
   PHASE(3);
   // P2: exclusive scan of cell counts -> slot starts; sentinel, clear flag, count the rebuild. Where every replica is a
   // few chunks of 1024 cells a block scans a replica, chunk after chunk; else in three phases: (a) chunk-local scans,
