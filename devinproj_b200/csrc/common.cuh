@@ -89,8 +89,9 @@ __device__ __forceinline__ void image3(double& dx, double& dy, double& dz, const
   }
 }
 
-// 1/x for normal positive x by Newton-Raphson from the hardware's FP64 reciprocal approximation (about 20 bits): two
-// quadratic steps, the second's residual exact in its FMA, leave under 1 ulp. x = 0 gives NaN through inf * 0.
+// 1/x for normal positive x by Newton-Raphson from the hardware's FP64 reciprocal approximation (about 20 bits): after the
+// first quadratic step (40 bits) the second's residual is exact in its FMA, so the result is the rounded reciprocal but for
+// ties. x = 0 gives NaN through inf * 0.
 __device__ __forceinline__ double recip(double x) {
   double y;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
@@ -98,13 +99,26 @@ __device__ __forceinline__ double recip(double x) {
   return fma(fma(-x, y, 1.0), y, y);
 }
 
-// 1/sqrt(x) for normal positive x: the hardware approximation (about 20 bits) and one step of the third-order iteration
-// y (1 + e/2 + 3 e^2/8), e = 1 - x y^2; within 2 ulp.
-__device__ __forceinline__ double recip_sqrt(double x) {
+// sqrt(x) and its reciprocal by Goldschmidt's coupled iteration (Markstein, "Software division and square root using
+// Goldschmidt's algorithms", 2004) from the hardware's FP64 approximation (about 20 bits): one step gives 39 bits of both,
+// then a residual that is exact in its FMA finishes each, so the root is the IEEE one and ir the rounded reciprocal of
+// that root, but for ties. Two results for 10 operations. Zero, subnormal and huge x (rare) take the IEEE operations.
+static __device__ __noinline__ double sqrt_recip_ieee(double x, double& ir) {
+  const double r = sqrt(x);
+  ir = 1.0 / r;
+  return r;
+}
+__device__ __forceinline__ double sqrt_recip(double x, double& ir) {
+  if ((unsigned)(__double2hiint(x) - 0x08000000) >= 0x70000000u) return sqrt_recip_ieee(x, ir);   // not in 2^[-895, 897)
   double y;
   asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  const double e = fma(-x * y, y, 1.0);
-  return fma(fma(0.375, e, 0.5), y * e, y);
+  double g = x * y, h = 0.5 * y;
+  const double e = fma(-g, h, 0.5);
+  g = fma(g, e, g);
+  h = fma(h, e, h);
+  const double r = fma(fma(-g, g, x), h, g), y1 = h + h;
+  ir = fma(fma(-r, y1, 1.0), y1, y1);
+  return r;
 }
 
 // The smallest double whose IEEE square root is at least r: r2 < square_reaching(r) decides as sqrt(r2) < r does.
@@ -115,44 +129,59 @@ inline double square_reaching(double r) {
   return t;
 }
 
-// erfc(x) and exp(-x^2) for x >= 0. (1 + 2x) exp(x^2) erfc(x) is a smooth function of t = (x - k) / (x + k) over the
-// whole half line (Shepherd and Laframboise, Math. Comp. 36, 1981): with k = 3.75 its Chebyshev series, computed here
-// in extended precision to degree 23 and summed as two chains in t^2, is within 5.5e-17; the result is within 3 ulp of
-// erfc (measured against 40 digits over [0, 8]). No ranges, so a warp's pairs stay together, and the exponential is the
-// one the forces need anyway: about half of the operations of erfc and exp apart.
-__device__ __forceinline__ double erfc_exp(double x, double& gauss) {
-  x = fmin(x, 1e3);   // both are zero from 39 on
-  const double s = x * x;
-  const double g = exp(-s);
-  gauss = fma(-g, fma(x, x, -s), g);   // the rounding of x^2
-  const double u = fma(2.0, x, 1.0), w = x + 3.75;
-  const double r = recip(u * w);
-  const double t = (x - 3.75) * u * r, t2 = t * t;
-  double a = -2.62310734713347593e-09;
-  a = fma(a, t2, 3.19792667166680421e-08);
-  a = fma(a, t2, -2.48571262480167447e-07);
-  a = fma(a, t2, 1.74198215862248163e-06);
-  a = fma(a, t2, -1.14380480333468935e-05);
-  a = fma(a, t2, 5.16465297417741622e-05);
-  a = fma(a, t2, 2.93714378044958009e-04);
-  a = fma(a, t2, -9.74657968326526208e-03);
-  a = fma(a, t2, -5.86933985766493402e-02);
-  a = fma(a, t2, -1.08803930142444619e-01);
-  a = fma(a, t2, 3.58541548547902569e-03);
-  a = fma(a, t2, 1.23751263083782748e+00);
-  double b = 3.11143338097992545e-10;
-  b = fma(b, t2, -3.74421008096201827e-09);
-  b = fma(b, t2, 2.32635087088591238e-08);
-  b = fma(b, t2, -5.72182306032240859e-08);
-  b = fma(b, t2, -9.73559896736774970e-07);
-  b = fma(b, t2, 2.23842391550822306e-05);
-  b = fma(b, t2, -2.90154080540841724e-04);
-  b = fma(b, t2, 1.75562585289529543e-03);
-  b = fma(b, t2, 2.83622774189564060e-02);
-  b = fma(b, t2, 9.23043211603774838e-02);
-  b = fma(b, t2, 8.22767384901452042e-02);
-  b = fma(b, t2, -1.40240598585546966e-01);
-  return fma(b, t, a) * (w * r) * gauss;
+// erfc(x) and exp(-x^2), x = alpha r >= 0, from a Chebyshev series of exp(x^2) erfc(x) over the whole half line in a rational
+// variable (the method of Shepherd and Laframboise, Math. Comp. 36, 1981). Here the variable vanishes with x: with
+// s = x / (x + 2), exp(x^2) erfc(x) (x + 2) = 2 + s h(s), and h, computed in 50 digits to degree 24 over [0, 27.5] (the
+// exponential is zero beyond), is within 1.4e-16, its coefficients' rounding. Below x = 0.6 the same h is summed as
+// 1 + s (h / (x + 2) - 1), whose error goes to half a unit with x; above, as (2 + s h) / (x + 2).
+// Its error in units of 2^-53 (10^5 points per range against quad precision, of this code transcribed with libm's
+// exponential): root mean square 0.5 at x -> 0, 1.3 up to 2.4, 1.5 up to 5; largest 5.1 and 6.3, and 9 on the tail beyond.
+// A series in (x - 3.75) / (x + 3.75) took the rounding of its argument near x = 0 (1.9, largest 7.2).
+// The product alpha r is rounded too, a relative error that erfc and the exponential take 2 x^2 fold: its low part goes
+// into the exponential for three operations. The force of one DSF pair (alpha rc = 2.4) is off by 1.6 to 1.8 units of its
+// terms at all distances up to 0.8 rc, against 1.6 to 2.8 with erfc and exp of the rounded product, and 1.7 to 3.7 with the
+// series above; of one Ewald pair (alpha rc = 4) by 1.2 to 1.6, against 1.3 to 8.9 and 1.6 to 15.
+// One set of coefficients and no branch on ranges, so a warp's pairs stay together, and the exponential is the one the
+// forces need anyway. 8000 ions' Ewald sum 418 -> 441 us, the 4096-ion force call 144.4 -> 146.3 us with this and
+// sqrt_recip, for the accuracy.
+__device__ __forceinline__ double erfc_exp(double alpha, double r, double& gauss) {
+  double x = alpha * r;
+  x = __double2hiint(x) < 0x408f4000 ? x : 1e3;   // both are zero from 39 on
+  const double x2 = x * x;
+  const double g = exp(-x2);
+  // the roundings of alpha r (whose 2 x^2 fold is the largest error of a distant pair) and of x^2
+  gauss = fma(-g, fma(x + x, fma(alpha, r, -x), fma(x, x, -x2)), g);
+  const double w = recip(x + 2.0), s = x * w;
+  const double t = fma(2.1454545454545455, s, -1.0), t2 = t * t;   // s in [0, 27.5 / 29.5] to [-1, 1]
+  double a = -7.03276698885457419e-10;
+  a = fma(a, t2, 3.69827855338635472e-09);
+  a = fma(a, t2, 4.27993055151075388e-09);
+  a = fma(a, t2, -9.77940454227550041e-08);
+  a = fma(a, t2, 3.31218823208566288e-07);
+  a = fma(a, t2, 3.32783527978017621e-07);
+  a = fma(a, t2, -8.39035049546208681e-06);
+  a = fma(a, t2, 4.51999891448717694e-05);
+  a = fma(a, t2, -1.37057017009071884e-04);
+  a = fma(a, t2, 3.94944399220502703e-05);
+  a = fma(a, t2, 3.03160715558250648e-03);
+  a = fma(a, t2, -1.16325487326915597e-02);
+  a = fma(a, t2, -1.99641985249578879e+00);
+  double b = -1.57096167960187793e-09;
+  b = fma(b, t2, 1.41665436886721111e-08);
+  b = fma(b, t2, -4.57254387984705977e-08);
+  b = fma(b, t2, -2.97566004091487844e-08);
+  b = fma(b, t2, 8.57659805297907151e-07);
+  b = fma(b, t2, -3.35487926425173185e-06);
+  b = fma(b, t2, 6.31148301325306036e-07);
+  b = fma(b, t2, 7.58170834748642645e-05);
+  b = fma(b, t2, -6.65704094465739086e-04);
+  b = fma(b, t2, 4.75080620679196094e-03);
+  b = fma(b, t2, -4.10826625607029136e-02);
+  b = fma(b, t2, 5.45359367176469600e-01);
+  const double h = fma(b, t, a);
+  const bool small = __double2hiint(x) < 0x3fe33333;   // x < 0.6
+  const double f = small ? fma(s, fma(h, w, -1.0), 1.0) : w * fma(s, h, 2.0);
+  return f * gauss;
 }
 
 // An atom's position and one more value (species or charge) as one 32-byte sector, read by one 256-bit load: a pair

@@ -915,9 +915,10 @@ __global__ void __launch_bounds__(kBlock, 4) k_dsf64(const Packed* __restrict__ 
       for (int x = xs; x < xe; ++x) excluded |= ex_idx[x] == j;
       if (excluded) continue;
       const double qq = qi * o.w;
-      const double ir = recip_sqrt(r2), r = r2 * ir;
+      double ir;
+      const double r = sqrt_recip(r2, ir);
       double gauss;
-      const double er = erfc_exp(P.a * r, gauss) * ir;
+      const double er = erfc_exp(P.a, r, gauss) * ir;
       v[3] = fma(qq, er - P.erc_rc + P.fshift * (r - P.rc), v[3]);
       const double fv = qq * (fma(fma(P.c, gauss, er), ir, -P.fshift) * ir);
       v[0] = fma(-fv, dx, v[0]);

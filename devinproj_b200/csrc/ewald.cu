@@ -215,10 +215,11 @@ __global__ void __launch_bounds__(kBlock) k_sfac_sum(const double2* __restrict__
 
 // One real-space pair: the force of j on i over d, coef (f_i -= coef d), and its energy without the charges' product.
 __device__ __forceinline__ double ewald_pair(const EwaldPar& P, double r2, double qq, double& er) {
-  const double ir = recip_sqrt(r2);
-  double gauss;
-  er = erfc_exp(P.a * (r2 * ir), gauss) * ir;
-  return qq * fma(P.c2a, gauss, er) * (ir * ir);
+  double ir, gauss;
+  const double r = sqrt_recip(r2, ir);
+  er = erfc_exp(P.a, r, gauss) * ir;
+  const double i2 = ir * ir, ir2 = fma(fma(-r2, i2, 1.0), i2, i2);   // 1/r^2 without the rounding of r twice
+  return qq * fma(P.c2a, gauss, er) * ir2;
 }
 
 // Real space, every pair once: a block takes 8 tiles of 32 atoms (a tile per warp, an atom per lane) against every

@@ -1,0 +1,107 @@
+"""Single pair terms of the FP64 kernels against 40 digits: the force of one pair (a dimer, two ions far from the others)
+is its term, so no sum averages the term's error.
+
+The tolerance is the root mean square error of the plain FP64 expression (IEEE square root and division, libm's erfc and
+exp) on the same distances, per range of distance, and on top of it, where the term holds them, that of an erfc and an
+exponential that are 1.5 units of 2^-53 off: the root mean square bound stated at `erfc_exp`."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+UNIT = 2.0 ** -53
+EDGES = np.array([1e-3, 0.1, 0.3, 0.6, 1.0])   # of the cutoff
+
+
+def _rms(error, r, rc):
+    return np.array([np.sqrt(np.mean(error[(r >= a * rc) & (r < b * rc)] ** 2)) for a, b in zip(EDGES, EDGES[1:])]) / UNIT
+
+
+def _dimers(torch, r):
+    """2 m atoms: the pair (2 k, 2 k + 1) at distance r[k] on the x axis, each listing the other only."""
+    n = 2 * len(r)
+    pos = np.zeros((n, 3))
+    pos[1::2, 0] = r
+    nbr = torch.zeros((n + 31) // 32 * 32, dtype=torch.int32)
+    nbr[:n] = torch.arange(n, dtype=torch.int32) ^ 1
+    return torch.from_numpy(pos).cuda(), nbr.cuda(), torch.ones(n, dtype=torch.int32, device="cuda")
+
+
+def _exact(r, alpha, rc):
+    """erfc(alpha r) / r, the force of it, and the shift at rc, to 40 digits."""
+    import mpmath as mp
+    with mp.workdps(40):
+        a, c = mp.mpf(alpha), 2 * mp.mpf(alpha) / mp.sqrt(mp.pi)
+        u = [mp.erfc(a * mp.mpf(x)) / mp.mpf(x) for x in r]
+        f = [y / mp.mpf(x) + c * mp.exp(-(a * mp.mpf(x)) ** 2) / mp.mpf(x) for x, y in zip(r, u)]
+        shift = mp.erfc(a * rc) / mp.mpf(rc) ** 2 + c * mp.exp(-(a * rc) ** 2) / rc
+    return u, f, shift
+
+
+def _relative(got, exact, scale):
+    import mpmath as mp
+    with mp.workdps(40):
+        return np.array([float((mp.mpf(float(g)) - e) / s) for g, e, s in zip(got, exact, scale)])
+
+
+@pytest.mark.parametrize("alpha,rc", [(0.0, 3.0), (0.2, 12.0), (0.8, 3.0), (1.9, 3.0)])
+def test_dsf_pair(alpha, rc):
+    from scipy.special import erfc
+    import torch
+
+    from devinproj_b200 import _lib
+    from devinproj_b200.device import stream_handle
+    L = _lib.lib()
+    rng = np.random.default_rng(5)
+    r = np.concatenate([rng.uniform(a * rc, b * rc, 1500) for a, b in zip(EDGES, EDGES[1:])])
+    pos, nbr, nnb = _dimers(torch, r)
+    n = len(pos)
+    q = torch.ones(n, dtype=torch.float64, device="cuda")
+    force, energy = torch.empty_like(pos), torch.empty(1, dtype=torch.float64, device="cuda")
+    work = torch.empty(L.acs_force_work_bytes(n), dtype=torch.uint8, device="cuda")
+    assert L.acs_dsf_fp64(pos.data_ptr(), q.data_ptr(), n, None, 0, nbr.data_ptr(), nnb.data_ptr(), 1, None, None, alpha, rc,
+                          1.0, force.data_ptr(), energy.data_ptr(), work.data_ptr(), work.numel(), stream_handle()) == 0
+    _, f, shift = _exact(r, alpha, rc)
+    c, erc = 2 * alpha / np.sqrt(np.pi), erfc(alpha * rc)
+    root = np.sqrt(r * r)
+    ir, ar = 1.0 / root, alpha * root
+    plain = ((erfc(ar) * (ir * ir) + c * np.exp(-(ar * ar)) * ir) - (erc / (rc * rc) + c * np.exp(-(alpha * rc) ** 2) / rc)) * ir * r
+    exact, scale = [x - shift for x in f], [x + shift for x in f]
+    want = _rms(_relative(plain, exact, scale), r, rc)
+    got = _rms(_relative(force[1::2, 0].cpu().numpy(), exact, scale), r, rc)
+    print(got, want)
+    assert np.all(got <= 1.05 * np.sqrt(want ** 2 + (1.5 if alpha else 0.0) ** 2))
+
+
+def test_ewald_pair():
+    """Two ions, the reciprocal weights zero: the force and the energy are one real-space term."""
+    from scipy.special import erfc
+    import torch
+
+    from devinproj_b200 import ewald
+    from devinproj_b200.device import stream_handle
+    L = ewald._bind()
+    rng = np.random.default_rng(6)
+    rc = 20.0
+    alpha = 4 / rc
+    r = np.concatenate([rng.uniform(a * rc, b * rc, 500) for a, b in zip(EDGES, EDGES[1:])])
+    pos = _dimers(torch, r)[0].reshape(-1, 2, 3).contiguous()
+    box = np.array([50.0, 60.0, 70.0])
+    q, kw = torch.ones(2, dtype=torch.float64, device="cuda"), torch.zeros(1, dtype=torch.float64, device="cuda")
+    kv = torch.tensor([[0.1, 0.2, 0.3]], dtype=torch.float64, device="cuda")
+    force = torch.empty_like(pos)
+    energy = torch.empty((len(r), 3), dtype=torch.float64, device="cuda")
+    work = torch.empty(L.acs_ewald_work_bytes(2, 1), dtype=torch.uint8, device="cuda")
+    for k in range(len(r)):
+        assert L.acs_ewald_fp64(pos[k].data_ptr(), q.data_ptr(), 2, box.ctypes.data, kv.data_ptr(), kw.data_ptr(), 1, alpha, rc,
+                                1.0, force[k].data_ptr(), energy[k].data_ptr(), work.data_ptr(), work.numel(),
+                                stream_handle()) == 0
+    u, f, _ = _exact(r, alpha, rc)
+    root = np.sqrt(r * r)
+    er = erfc(alpha * root) / root
+    plain = (er + 2 * alpha / np.sqrt(np.pi) * np.exp(-(alpha * root) ** 2)) / (r * r) * r
+    for got, expr, exact in ((force[:, 1, 0], plain, f), (energy[:, 0], er, u)):
+        want = _rms(_relative(expr, exact, exact), r, rc)
+        have = _rms(_relative(got.cpu().numpy(), exact, exact), r, rc)
+        print(have, want)
+        assert np.all(have <= 1.05 * np.sqrt(want ** 2 + 1.5 ** 2))
