@@ -790,7 +790,9 @@ __global__ void __launch_bounds__(kBlock, 4) k_lj64(const double* __restrict__ p
         const double w = fma(sr6, sr6, -sr6);
         v[3] = ONE ? v[3] + w : fma(e, w, v[3]);
         if (in) cnt += e;
-        const double c = (ONE ? ir2 : e * ir2) * fma(sr6, sr6, w);
+        // 2 sr6^2 - sr6 in one rounding: formed from w it took two, and one pair's force was up to 6% further off (root
+        // mean square, 1.06 against 0.99 units of 2^-53 of its terms at 1.2 to 1.5 sigma)
+        const double c = (ONE ? ir2 : e * ir2) * fma(sr6 + sr6, sr6, -sr6);
         if (in) {   // not 0 * d: an atom that is not finite has no neighbours and must not reach their sums
           v[0] = fma(c, d[q][0], v[0]);
           v[1] = fma(c, d[q][1], v[1]);

@@ -73,6 +73,38 @@ def test_dsf_pair(alpha, rc):
     assert np.all(got <= 1.05 * np.sqrt(want ** 2 + (1.5 if alpha else 0.0) ** 2))
 
 
+def test_lj_pair():
+    """Against the plain expression with the product-difference 2 s^2 - s in one FMA (here in extended precision), which is
+    the same number of roundings: 2% for the sampling of rare differences."""
+    import torch
+
+    from devinproj_b200 import _lib
+    from devinproj_b200.device import stream_handle
+    L = _lib.lib()
+    rng = np.random.default_rng(7)
+    bins = np.array([0.8, 1.0, 1.2, 1.5, 2.0, 2.5])
+    r = np.concatenate([rng.uniform(a, b, 40000) for a, b in zip(bins, bins[1:])])
+    pos, nbr, nnb = _dimers(torch, r)
+    n = len(pos)
+    sp, one = torch.zeros(n, dtype=torch.int32, device="cuda"), np.ones(1)
+    force, energy = torch.empty_like(pos), torch.empty(1, dtype=torch.float64, device="cuda")
+    work = torch.empty(L.acs_force_work_bytes(n), dtype=torch.uint8, device="cuda")
+    assert L.acs_lj_fp64(pos.data_ptr(), sp.data_ptr(), n, None, 0, nbr.data_ptr(), nnb.data_ptr(), 1, 1, one.ctypes.data,
+                         one.ctypes.data, 2.5, force.data_ptr(), energy.data_ptr(), work.data_ptr(), work.numel(),
+                         stream_handle()) == 0
+    ext = r.astype(np.longdouble)
+    exact, terms = 24 * (2 * ext ** -12 - ext ** -6) / ext, 24 * (2 * ext ** -12 + ext ** -6) / ext
+    ir2 = 1.0 / (r * r)
+    s6 = ir2 * ir2 * ir2
+    plain = 24 * ((2 * s6).astype(np.longdouble) * s6 - s6).astype(float) * ir2 * r
+    for a, b in zip(bins, bins[1:]):
+        k = (r >= a) & (r < b)
+        got, want = (np.sqrt(np.mean(((x - exact) / terms)[k].astype(float) ** 2)) / UNIT
+                     for x in (force[1::2, 0].cpu().numpy(), plain))
+        print(a, b, got, want)
+        assert got <= 1.02 * want
+
+
 def test_ewald_pair():
     """Two ions, the reciprocal weights zero: the force and the energy are one real-space term."""
     from scipy.special import erfc
