@@ -137,3 +137,36 @@ def test_ewald_pair():
         have = _rms(_relative(got.cpu().numpy(), exact, exact), r, rc)
         print(have, want)
         assert np.all(have <= 1.05 * np.sqrt(want ** 2 + 1.5 ** 2))
+
+
+def test_descriptor_pair():
+    """One neighbour: a vector feature is g fc(r) / r, the same number for the three axes, times the FP32 component of d,
+    rounded once. So V_x / d_x and V_y / d_y differ by at most two roundings, 2^-23."""
+    import torch
+
+    from devinproj_b200 import learned
+    from devinproj_b200.device import stream_handle
+    L = learned._bind()
+    rng = np.random.default_rng(8)
+    m = 2000
+    pos = np.zeros((2 * m, 3))
+    u = rng.normal(0, 1, (m, 3))
+    pos[1::2] = u / np.linalg.norm(u, axis=1)[:, None] * rng.uniform(1.5, 9.5, m)[:, None]
+    p, nbr, nnb = _dimers(torch, np.zeros(m))
+    p = torch.from_numpy(pos).cuda()
+    sp = torch.zeros(2 * m, dtype=torch.int32, device="cuda")
+    rbf = learned.rbf_params()
+    params = np.array([rbf["r0"], rbf["dmu"], 1 / (2 * rbf["s"] ** 2), rbf["rc"], 0, 0], dtype=np.float32)
+    mean, inv_std = torch.zeros(64, device="cuda"), torch.ones(64, device="cuda")
+    X = torch.empty((2 * m, 80), dtype=torch.bfloat16, device="cuda")
+    V = torch.empty((2 * m, 64, 3), device="cuda")
+    assert L.acs_descriptors(p.data_ptr(), sp.data_ptr(), 2 * m, None, 0, nbr.data_ptr(), nnb.data_ptr(), 1,
+                             params.ctypes.data, mean.data_ptr(), inv_std.data_ptr(), X.data_ptr(), V.data_ptr(),
+                             stream_handle()) == 0
+    d = pos[1::2].astype(np.float32).astype(np.float64)
+    q = V.cpu().numpy()[::2, :32].astype(np.float64) / d[:, None, :]
+    big = np.abs(V.cpu().numpy()[::2, :32]).min(2) > 1e-30   # no subnormal numbers among them
+    q = q[big]
+    spread = (q.max(1) - q.min(1)) / np.abs(q).mean(1)
+    print(len(spread), spread.max() * 2 ** 23)
+    assert len(spread) > m and spread.max() <= 2.0 ** -23 * (1 + 1e-6)
