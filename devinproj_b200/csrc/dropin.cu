@@ -369,6 +369,54 @@ __global__ void __launch_bounds__(kBlock) k_list_atoms(const double* __restrict_
   if (lane == 0) list_end(i, cnt, maxnb, nnb, status);
 }
 
+// Neighbour lists, a lane per atom in cell order, for cells with few atoms (sparse_cells): bound by the latency of a
+// stencil's cell starts and candidates, with up to 1024 atoms of an SM in flight. The same lists entry by entry. Whole build
+// of 10^6 atoms in random order at 0.2, 0.7 and 1.6 atoms a cell: 193, 214, 264 us; a warp per atom 930, 1184, 1297. The
+// stencil's starts read together into registers took 220, 283, 375 (104 registers).
+template <bool WRAP>
+__global__ void __launch_bounds__(kBlock) k_list_sparse(const double* __restrict__ pos, int64_t n,
+                                                        const __grid_constant__ GridDev g, Screen f,
+                                                        const int32_t* __restrict__ cell_of,
+                                                        const int32_t* __restrict__ start,
+                                                        const float4* __restrict__ screen, int maxnb,
+                                                        int32_t* __restrict__ nbr, int32_t* __restrict__ nnb,
+                                                        acs_dev_status* status) {
+  const int64_t slot = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (slot >= n) return;
+  const float4 me = screen[slot];
+  const int32_t i = __float_as_int(me.w);
+  int32_t* __restrict__ row = nbr + nbr_slot(i, 0, maxnb);
+  int cnt = 0;
+  const int c = cell_of[i];
+#pragma unroll 1
+  for (int st = 0; st < 18; ++st) {
+    int k0, len, im;
+    stencil_stretch(g, start, c, st, k0, len, im);
+    float mx = me.x, my = me.y, mz = me.z;
+    if (!WRAP) {
+      mx -= (float)(im % 3 - 1) * f.L[0];
+      my -= (float)((im / 3) % 3 - 1) * f.L[1];
+      mz -= (float)(im / 9 - 1) * f.L[2];
+    }
+    for (int k = k0; k < k0 + len; ++k) {
+      const float4 o = __ldg(screen + k);
+      float dx = o.x - mx, dy = o.y - my, dz = o.z - mz;
+      if (WRAP) {
+        dx -= f.L[0] * rintf(dx * f.inv[0]);
+        dy -= f.L[1] * rintf(dy * f.inv[1]);
+        dz -= f.L[2] * rintf(dz * f.inv[2]);
+      }
+      const float q = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
+      if (q >= f.hi || k == slot) continue;
+      const int32_t j = __float_as_int(o.w);
+      if (!(q <= f.lo) && !exact_pair(pos, i, j, g)) continue;
+      if (cnt < maxnb) row[(int64_t)cnt * 32] = j;
+      ++cnt;
+    }
+  }
+  list_end(i, cnt, maxnb, nnb, status);
+}
+
 // Neighbour lists, a warp per home cell (32 of its atoms at a time), for systems with cells enough to fill the chip: the
 // stencil's candidates are read, shifted to their image and culled against the home atoms' bounding box once for all
 // home atoms, packed to full batches of 32 in shared memory, and each batch is screened against two home atoms per
@@ -508,6 +556,22 @@ __global__ void __launch_bounds__(kBlock) k_list_cells(const double* __restrict_
   }
 }
 
+// One pair into the histogram below: its distance by the reference's FP64 expression and its bin by NumPy's rule.
+__device__ __forceinline__ void count_pair(const double* __restrict__ pos, const int32_t* __restrict__ sp, int64_t i, int64_t j,
+                                           const GridDev& g, int species, int bins, double rmax, double step, double per_bin,
+                                           unsigned int* sh_hist) {
+  double dx = sub(pos[3 * j], pos[3 * i]), dy = sub(pos[3 * j + 1], pos[3 * i + 1]), dz = sub(pos[3 * j + 2], pos[3 * i + 2]);
+  image3_any(dx, dy, dz, g.box);
+  const double r = __dsqrt_rn(norm2(dx, dy, dz));
+  if (r <= rmax && (species < 0 || sp[j] == species)) {
+    int idx = min((int)(r * per_bin), bins - 1);
+    if (r < mul((double)idx, step)) idx -= 1;
+    const double upper = idx + 1 == bins ? rmax : mul((double)(idx + 1), step);
+    if (r >= upper && idx != bins - 1) idx += 1;
+    atomicAdd(&sh_hist[idx], 1u);
+  }
+}
+
 // Pair-distance histogram of accusim/analysis.py:7-24 (rdf): pairs i < j, both of `species` (all when < 0),
 // minimum-image r by the reference's FP64 expression, binned by NumPy's uniform-bin rule on [0, rmax]
 // (numpy histogram: index = int((r / rmax) * bins), the right edge into the last bin, then one step down if
@@ -535,18 +599,7 @@ __global__ void __launch_bounds__(kBlock) k_rdf(const double* __restrict__ pos, 
   auto measure = [&](int m) {   // the first m queued pairs
     if (lane < m) {
       const int2 p = queue[wib][lane];
-      double dx = sub(pos[3 * (int64_t)p.y], pos[3 * (int64_t)p.x]),
-             dy = sub(pos[3 * (int64_t)p.y + 1], pos[3 * (int64_t)p.x + 1]),
-             dz = sub(pos[3 * (int64_t)p.y + 2], pos[3 * (int64_t)p.x + 2]);
-      image3_any(dx, dy, dz, g.box);
-      const double r = __dsqrt_rn(norm2(dx, dy, dz));
-      if (r <= rmax && (species < 0 || sp[p.y] == species)) {
-        int idx = min((int)(r * per_bin), bins - 1);
-        if (r < mul((double)idx, step)) idx -= 1;
-        const double upper = idx + 1 == bins ? rmax : mul((double)(idx + 1), step);
-        if (r >= upper && idx != bins - 1) idx += 1;
-        atomicAdd(&sh_hist[idx], 1u);
-      }
+      count_pair(pos, sp, p.x, p.y, g, species, bins, rmax, step, per_bin, sh_hist);
     }
   };
   for (int64_t slot = (int64_t)blockIdx.x * (kBlock / 32) + wib; slot < n; slot += (int64_t)gridDim.x * (kBlock / 32)) {
@@ -597,6 +650,77 @@ __global__ void __launch_bounds__(kBlock) k_rdf(const double* __restrict__ pos, 
     }
   }
   measure(queued);
+  __syncthreads();
+  for (int b = threadIdx.x; b < bins; b += blockDim.x)
+    if (sh_hist[b]) atomicAdd(&hist[b], (unsigned long long)sh_hist[b]);
+}
+
+// The same counts for cells with few atoms (sparse_cells): a lane per atom, each walking its own stencil, the pairs in the
+// warp's queue. 10^6 atoms at 0.2, 0.7 and 3.3 a cell: 191, 198, 294 us; a warp per atom 527, 676, 790; a lane per atom that
+// measured its own pairs at once, on divergent FP64 code, 312, 585, 1195.
+template <bool WRAP>
+__global__ void __launch_bounds__(kBlock) k_rdf_sparse(const double* __restrict__ pos, const int32_t* __restrict__ sp, int64_t n,
+                                                       const __grid_constant__ GridDev g, Screen f,
+                                                       const int32_t* __restrict__ cell_of,
+                                                       const int32_t* __restrict__ start,
+                                                       const float4* __restrict__ screen, int species, int bins, double rmax,
+                                                       double step, unsigned long long* __restrict__ hist) {
+  extern __shared__ unsigned int sh_hist[];
+  __shared__ int2 queue[kBlock / 32][64];
+  for (int b = threadIdx.x; b < bins; b += blockDim.x) sh_hist[b] = 0u;
+  __syncthreads();
+  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+  const unsigned below = (1u << lane) - 1u;
+  const double per_bin = bins / rmax;
+  int queued = 0;
+  for (int64_t base = (int64_t)blockIdx.x * blockDim.x + 32 * wib; base < n; base += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t slot = base + lane;
+    const float4 me = screen[min(slot, n - 1)];
+    const int32_t i = __float_as_int(me.w);
+    const bool on = slot < n && (species < 0 || sp[i] == species);
+    const int c = cell_of[i], c2 = c % g.nc[2];
+    const bool wraps = __any_sync(0xffffffffu, c2 == 0 || c2 == g.nc[2] - 1);
+#pragma unroll 1
+    for (int st = 0; st < 18; st += wraps ? 1 : 2) {
+      int k0, len, im;
+      stencil_stretch(g, start, c, st, k0, len, im);
+      const int end = on ? k0 + len : 0;
+      float mx = me.x, my = me.y, mz = me.z;
+      if (!WRAP) {
+        mx -= (float)(im % 3 - 1) * f.L[0];
+        my -= (float)((im / 3) % 3 - 1) * f.L[1];
+        mz -= (float)(im / 9 - 1) * f.L[2];
+      }
+      for (int k = (int)max((int64_t)k0, slot + 1); __any_sync(0xffffffffu, k < end); ++k) {   // later atoms only
+        float4 o = make_float4(3e30f, 3e30f, 3e30f, 0.f);
+        if (k < end) o = __ldg(screen + k);
+        float dx = o.x - mx, dy = o.y - my, dz = o.z - mz;
+        if (WRAP) {
+          dx -= f.L[0] * rintf(dx * f.inv[0]);
+          dy -= f.L[1] * rintf(dy * f.inv[1]);
+          dz -= f.L[2] * rintf(dz * f.inv[2]);
+        }
+        const bool maybe = k < end && !(fmaf(dz, dz, fmaf(dy, dy, dx * dx)) >= f.hi);
+        const unsigned bal = __ballot_sync(0xffffffffu, maybe);
+        if (maybe) queue[wib][queued + __popc(bal & below)] = make_int2(i, __float_as_int(o.w));
+        queued += __popc(bal);
+        __syncwarp();
+        if (queued >= 32) {
+          const int2 p = queue[wib][lane];
+          count_pair(pos, sp, p.x, p.y, g, species, bins, rmax, step, per_bin, sh_hist);
+          queued -= 32;
+          const int2 rest = queue[wib][32 + lane];
+          __syncwarp();
+          queue[wib][lane] = rest;
+          __syncwarp();
+        }
+      }
+    }
+  }
+  if (lane < queued) {
+    const int2 p = queue[wib][lane];
+    count_pair(pos, sp, p.x, p.y, g, species, bins, rmax, step, per_bin, sh_hist);
+  }
   __syncthreads();
   for (int b = threadIdx.x; b < bins; b += blockDim.x)
     if (sh_hist[b]) atomicAdd(&hist[b], (unsigned long long)sh_hist[b]);
@@ -1075,6 +1199,15 @@ int bin_cells(const double* pos, int64_t n, const acs_grid* g, void* work, cudaS
   return 0;
 }
 
+// Whether a lane per atom on its own stencil beats a warp per atom (k_list_sparse, k_rdf_sparse): where cells hold few
+// atoms, a warp's 32 lanes meet stretches of a few candidates, if there are atoms enough to fill the chip. List build, warp
+// against lane per atom, at 0.7 and 3.4 atoms a cell: 16,000 atoms 58, 58 against 53, 70 us; 32,000 76, 82 against 52, 66;
+// 250,000 322, 362 against 84, 123; 10^6 1184, 1338 against 214, 371 (a thread per atom testing every
+// candidate in FP64 499, 1184). At 4.6 a cell the warp per cell takes over (32,000 atoms 60 against 80). Histogram: 32,000
+// atoms 58, 63 against 58, 78; 64,000 79, 89 against 58, 85; 10^6 676, 790 against 198, 294 (in FP64 530, 1344).
+constexpr int64_t kSparseList = 20000, kSparseRdf = 50000;
+bool sparse_cells(int64_t n, int64_t nc, int64_t least) { return n >= least && n < 4 * nc; }
+
 }  // namespace
 
 // ===================================================================================== C ABI ==
@@ -1164,6 +1297,9 @@ int acs_nlist_build(const double* pos, int64_t n, const acs_grid* g, int32_t max
     const unsigned chunks = (unsigned)std::max<int64_t>(1, std::min<int64_t>(ceil_div(2 * n, 32 * nc), 64));
     k_list_cells<<<dim3((unsigned)ceil_div(nc, kBlock / 32), chunks), kBlock, 0, s>>>(pos, gd, f, nc, cb.start, cb.screen,
                                                                                      maxnb, nbr, nnb, status);
+  } else if (sparse_cells(n, nc, kSparseList)) {
+    (wrap ? k_list_sparse<true> : k_list_sparse<false>)<<<(int)ceil_div(n, kBlock), kBlock, 0, s>>>(
+        pos, n, gd, f, cb.cell_of, cb.start, cb.screen, maxnb, nbr, nnb, status);
   } else {
     // 4 loads in flight where a stretch of 3 cells fills them (4096 ions in 27 cells: 53 us with 1, 49 with 2, 45 with 4),
     // else 2 (8000 ions in 216 cells: 41, 36, 39)
@@ -1193,7 +1329,9 @@ int acs_rdf_hist(const double* pos, const int32_t* sp, int64_t n, const acs_grid
   const bool wrap = g->ncell[0] < 4 || g->ncell[1] < 4 || g->ncell[2] < 4;
   // one round of blocks (up to 4 on each of 148 SMs), so that a block's counts are added to the result once
   const int blocks = (int)std::min<int64_t>(592, ceil_div(n, kBlock / 32));
-  (wrap ? k_rdf<true> : k_rdf<false>)<<<blocks, kBlock, sizeof(unsigned int) * bins, s>>>(
+  const bool sparse = sparse_cells(n, grid_cells(g), kSparseRdf);
+  auto kernel = sparse ? (wrap ? k_rdf_sparse<true> : k_rdf_sparse<false>) : (wrap ? k_rdf<true> : k_rdf<false>);
+  kernel<<<blocks, kBlock, sizeof(unsigned int) * bins, s>>>(
       pos, sp, n, to_dev(g), screen_of(g, square_reaching(nextafter(rmax, HUGE_VAL))), cb.cell_of,
       cb.start, cb.screen, species, bins, rmax, rmax / bins, hist);
   return launch_status();
