@@ -808,8 +808,19 @@ struct PairSplit {
   int64_t blocks;
 };
 
-// The fewest phases (at most 32) that give `threads`, then more while each thread keeps kPhaseEntries of the `entries`
-// an atom has room for, up to kMostThreads in all. 151,552 threads are resident, so a split below that leaves places
+// About how many neighbours an atom has in its list (all atoms without one), from the density and the cutoff alone: the
+// split decides the order of an atom's sum, which must not depend on the buffer the caller gave the list (its capacity).
+// A list holds the neighbours to the cutoff plus a skin, 1.4 times those inside in the usual 0.3 of 2.5. Without a box: no
+// statement (infinite).
+double pairs_per_atom(int64_t n, bool list, const double* box3, double rc) {
+  if (!list) return (double)n;
+  if (!box3) return HUGE_VAL;
+  const double V = fabs(box3[0] * box3[1] * box3[2]);
+  return V > 0.0 ? std::min((double)n, 1.4 * 4.0 / 3.0 * M_PI * rc * rc * rc * ((double)n / V)) : (double)n;
+}
+
+// The fewest phases (at most 32) that give `threads`; then, if `spread`, more while each thread keeps kPhaseEntries
+// of an atom's pairs, up to kMostThreads in all. 151,552 threads are resident, so a split below that leaves places
 // empty, one of a few waves loses its last one, and a thread with few entries is all prologue. DSF terms are long enough
 // to want several waves: 32,768 ions 141 us at 131,072 threads, 118 at 262,144, 112 at 524,288; 175,616 ions 678, 595,
 // 544; 64,000 ions 224, 213, 205 (209 at 1,048,576). LJ with 79 entries an atom does not: 32,000 atoms 18.5 us at
@@ -817,13 +828,13 @@ struct PairSplit {
 // 1,048,576 atoms 0.355 ms with one phase, 0.372 with two, 0.430 with four. With 351 entries it does: 110,592 ions
 // 135 us with four phases, 157 with two, 147 with eight; 175,616 ions 210 with four, 300 with one.
 constexpr int64_t kMostThreads = 1 << 20, kLjThreads = 98304, kDsfThreads = 524288;
-constexpr int kPhaseEntries = 80;
-PairSplit pair_split(int64_t n, int64_t threads, int64_t entries) {
+constexpr double kPhaseEntries = 56.0;
+PairSplit pair_split(int64_t n, int64_t threads, double pairs, bool spread) {
   PairSplit s;
   s.log2_phases = 0;
   while (s.log2_phases < 5 && (n << s.log2_phases) < threads) ++s.log2_phases;
-  while (s.log2_phases < 5 && (n << (s.log2_phases + 1)) <= kMostThreads &&
-         entries >> (s.log2_phases + 1) >= kPhaseEntries)
+  while (spread && pairs < HUGE_VAL && s.log2_phases < 5 && (n << (s.log2_phases + 1)) <= kMostThreads &&
+         pairs >= kPhaseEntries * (2 << s.log2_phases))
     ++s.log2_phases;
   s.atoms = kBlock >> s.log2_phases;
   s.blocks = ceil_div(n, s.atoms);
@@ -977,15 +988,22 @@ __global__ void __launch_bounds__(kBlock, 4) k_lj64(const double* __restrict__ p
 
 template <bool PACKED, bool ONE>
 void launch_lj64(const double* pos, const int32_t* sp, const Packed* pk, int64_t n, const ImageBox& b, const int32_t* nbr,
-                 const int32_t* nnb, int maxnb, const LJTab& t, double* force, double* partials, unsigned int* ticket,
-                 double* energy, cudaStream_t s) {
-  const PairSplit split = pair_split(n, kLjThreads, nbr ? maxnb : n);
+                 const int32_t* nnb, int maxnb, const LJTab& t, const PairSplit& split, double* force, double* partials,
+                 unsigned int* ticket, double* energy, cudaStream_t s) {
   if (nbr)
     k_lj64<false, PACKED, ONE><<<(int)split.blocks, kBlock, 0, s>>>(pos, sp, pk, n, b, nbr, nnb, maxnb, t, split, force,
                                                                     partials, ticket, energy);
   else
     k_lj64<true, PACKED, ONE><<<(int)split.blocks, kBlock, 0, s>>>(pos, sp, pk, n, b, nullptr, nullptr, 0, t, split,
                                                                    force, partials, ticket, energy);
+}
+
+PairSplit lj_split(int64_t n, bool list, const double* box3, int n_species, const double* eps_tab, const double* sig_tab,
+                   double cutoff) {
+  double sig = 0.0;   // the largest of a pair that interacts
+  for (int a = 0; a < n_species * n_species; ++a)
+    if (eps_tab[a] > 0.0) sig = std::max(sig, sig_tab[a]);
+  return pair_split(n, kLjThreads, pairs_per_atom(n, list, box3, cutoff * sig), true);
 }
 
 LJTab lj_tables(int n_species, const double* eps_tab, const double* sig_tab, double cutoff) {
@@ -1406,11 +1424,12 @@ int acs_lj_fp64(const double* pos, const int32_t* sp, int64_t n, const double* b
   int st = force_setup(pos, sp, nullptr, n, work, work_bytes, &partials, &ticket, &pk, s);
   if (st) return st;
   const LJTab t = lj_tables(n_species, eps_tab, sig_tab, cutoff);
+  const PairSplit split = lj_split(n, nbr, box3, n_species, eps_tab, sig_tab, cutoff);
   const ImageBox b = image_box(box3, periodic);
   if (n_species == 1)
-    launch_lj64<true, true>(pos, sp, pk, n, b, nbr, nnb, maxnb, t, force, partials, ticket, energy_dev, s);
+    launch_lj64<true, true>(pos, sp, pk, n, b, nbr, nnb, maxnb, t, split, force, partials, ticket, energy_dev, s);
   else
-    launch_lj64<true, false>(pos, sp, pk, n, b, nbr, nnb, maxnb, t, force, partials, ticket, energy_dev, s);
+    launch_lj64<true, false>(pos, sp, pk, n, b, nbr, nnb, maxnb, t, split, force, partials, ticket, energy_dev, s);
   return launch_status();
 }
 
@@ -1438,7 +1457,7 @@ int acs_dsf_fp64(const double* pos, const double* q, int64_t n, const double* bo
   P.fshift = P.erc / (rcut * rcut) + P.c * exp(-((alpha * rcut) * (alpha * rcut))) / rcut;
   P.self_coef = P.erc / (2.0 * rcut) + alpha / sqrt(M_PI);
   const ImageBox b = image_box(box3, periodic);
-  const PairSplit split = pair_split(n, kDsfThreads, 0);
+  const PairSplit split = pair_split(n, kDsfThreads, pairs_per_atom(n, nbr, box3, rcut), false);
   if (nbr)
     k_dsf64<false><<<(int)split.blocks, kBlock, 0, s>>>(pk, n, b, nbr, nnb, maxnb, ex_start, ex_idx, P, split, force,
                                                        partials, ticket, energy_dev);
@@ -1590,10 +1609,11 @@ extern "C" int acs_lj_fp64_noalloc(const double* pos, const int32_t* sp, int64_t
   unsigned int* ticket = (unsigned int*)((char*)scratch + kNoAllocMaxBlocks * 8);
   if (cudaMemsetAsync(ticket, 0, 4, s) != cudaSuccess) return ACS_ERR_CUDA;
   const LJTab t = lj_tables(n_species, eps_tab, sig_tab, cutoff);
+  const PairSplit split = lj_split(n, nbr, box3, n_species, eps_tab, sig_tab, cutoff);
   const ImageBox b = image_box(box3, periodic);
   if (n_species == 1)   // the same arithmetic as acs_lj_fp64, bit for bit
-    launch_lj64<false, true>(pos, sp, nullptr, n, b, nbr, nnb, maxnb, t, force, partials, ticket, energy_dev, s);
+    launch_lj64<false, true>(pos, sp, nullptr, n, b, nbr, nnb, maxnb, t, split, force, partials, ticket, energy_dev, s);
   else
-    launch_lj64<false, false>(pos, sp, nullptr, n, b, nbr, nnb, maxnb, t, force, partials, ticket, energy_dev, s);
+    launch_lj64<false, false>(pos, sp, nullptr, n, b, nbr, nnb, maxnb, t, split, force, partials, ticket, energy_dev, s);
   return launch_status();
 }

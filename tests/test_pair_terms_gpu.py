@@ -170,3 +170,31 @@ def test_descriptor_pair():
     spread = (q.max(1) - q.min(1)) / np.abs(q).mean(1)
     print(len(spread), spread.max() * 2 ** 23)
     assert len(spread) > m and spread.max() <= 2.0 ** -23 * (1 + 1e-6)
+
+
+# 110,592 atoms with 250 pairs each (several threads per atom there, by the rule's second part) and 13,824 with 55
+@pytest.mark.parametrize("n_side,rc", [(48, 4.1), (24, 2.5)])
+def test_lj_bits_do_not_depend_on_the_list_capacity(n_side, rc):
+    """The same list in buffers of three capacities: the same force and energy, bit for bit, as after a regrow on overflow."""
+    import torch
+
+    from tests.test_fp64_kernels_gpu import _abi, _build_list, _grid
+    _, L, st = _abi()
+    rng = np.random.default_rng(n_side)
+    n = n_side ** 3
+    box = np.array([1.0, 1.0, 1.0]) * (n / 0.8442) ** (1 / 3)
+    grid = np.stack(np.meshgrid(*[np.arange(n_side)] * 3, indexing="ij"), -1).reshape(-1, 3)
+    pos = torch.from_numpy((grid + 0.5 + rng.normal(0, 0.05, (n, 3))) * box / n_side % box).cuda()
+    sp, one = torch.zeros(n, dtype=torch.int32, device="cuda"), np.ones(1)
+    g = _grid(L, box, 1.12 * rc)
+    work = torch.empty(L.acs_force_work_bytes(n), dtype=torch.uint8, device="cuda")
+    expected = int(4 / 3 * np.pi * (1.12 * rc) ** 3 * 0.8442)
+    out = []
+    for maxnb in (expected + 40, 2 * expected + 40, 4 * expected):
+        nbr, nnb = _build_list(torch, L, st, pos, g, maxnb)
+        force, energy = torch.empty_like(pos), torch.empty(1, dtype=torch.float64, device="cuda")
+        assert L.acs_lj_fp64(pos.data_ptr(), sp.data_ptr(), n, box.ctypes.data, 1, nbr.data_ptr(), nnb.data_ptr(), maxnb, 1,
+                             one.ctypes.data, one.ctypes.data, rc, force.data_ptr(), energy.data_ptr(), work.data_ptr(),
+                             work.numel(), st) == 0
+        out.append(torch.cat([force.reshape(-1), energy]).cpu())
+    assert torch.equal(out[0], out[1]) and torch.equal(out[0], out[2])
