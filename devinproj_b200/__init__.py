@@ -6,25 +6,16 @@ whose state stays on the GPU; `to_gpu`, which moves a simulation built by accusi
 and `GpuSimulation`, the device-resident engine (FP32-compensated pairs, FP64
 state, CUDA-graph step loops, batched replicas). All compute is hand-written CUDA in libaccusim_b200.so.
 """
-try:
-    from . import _accusim  # noqa: F401  (accusim, the host framework)
-except ImportError as _e:   # the build script and the C-ABI binding (`_lib`) work without it, the plug-ins do not
-    _missing = str(_e)
-
-    def __getattr__(name):
-        if name in __all__:
-            raise ImportError(_missing)
-        raise AttributeError(f"module {__name__!r} has no attribute {name!r}")
-else:
-    from .analysis import rdf
-    from .convert import gpu_twin, to_gpu
-    from .engine import GpuSimulation
-    from .ensemble import ReplicaEnsemble, calibrate_dt_ensemble, richardson_ensemble
-    from .ewald import Ewald
-    from .forces import DampedShiftedCoulomb, LennardJones, VerletList, cell_list_pairs
-    from .integrators import Langevin, NoseHoover, VelocityVerlet
-    from .learned import LearnedCorrection
-    from .state import GpuSystem
+from . import _accusim  # noqa: F401  (accusim, the host framework)
+from .analysis import rdf
+from .convert import gpu_twin, to_gpu
+from .engine import GpuSimulation
+from .ensemble import ReplicaEnsemble, calibrate_dt_ensemble, richardson_ensemble
+from .ewald import Ewald
+from .forces import DampedShiftedCoulomb, LennardJones, VerletList, cell_list_pairs
+from .integrators import Langevin, NoseHoover, VelocityVerlet
+from .learned import LearnedCorrection
+from .state import GpuSystem
 
 __all__ = ["DampedShiftedCoulomb", "Ewald", "GpuSimulation", "GpuSystem", "Langevin", "LearnedCorrection",
            "LennardJones", "NoseHoover", "ReplicaEnsemble", "VelocityVerlet", "VerletList", "calibrate_dt_ensemble",

@@ -5,6 +5,10 @@ The GPU classes of this package subclass accusim's own `Force` and `Integrator` 
 (accusim/accuracy.py:149, accusim/advisor.py:36) see the reference classes. accusim is pure Python; it is
 imported from the environment, or else from the repository's own offline install under `baseline/_ref`
 (made by `baseline/install_reference.sh`).
+
+Without accusim `accusim` is None here. The build script, the C-ABI bindings and the engine below the plug-ins need
+nothing of it, so every module still imports; a class of accusim, or one derived from it, raises ImportError when an
+object of it is made.
 """
 from __future__ import annotations
 
@@ -12,22 +16,38 @@ import os
 import sys
 
 _REPO_INSTALL = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "baseline", "_ref")
+MISSING = ("devinproj_b200 plugs into the accusim package, which is not importable: install it "
+           "(pip install <accusim checkout>, or baseline/install_reference.sh)")
 
 try:
-    import accusim  # noqa: F401
+    import accusim
 except ImportError:
+    accusim = None
     if os.path.isdir(os.path.join(_REPO_INSTALL, "accusim")):
         sys.path.append(_REPO_INSTALL)
-        import accusim  # noqa: F401
-    else:
-        raise ImportError("devinproj_b200 plugs into the accusim package, which is not importable: install it "
-                          "(pip install <accusim checkout>, or baseline/install_reference.sh)") from None
+        import accusim
 
-import accusim.accuracy as accuracy  # noqa: E402
-import accusim.forces as forces  # noqa: E402
-import accusim.integrators as integrators  # noqa: E402
-import accusim.simulation as simulation  # noqa: E402
-import accusim.system as system  # noqa: E402
-import accusim.units as units  # noqa: E402
+if accusim is not None:
+    import accusim.accuracy as accuracy
+    import accusim.forces as forces
+    import accusim.integrators as integrators
+    import accusim.simulation as simulation
+    import accusim.system as system
+    import accusim.units as units
+else:
+    def _refuse(cls, *args, **kwargs):
+        raise ImportError(MISSING)
+
+    class _Absent:
+        """A module of accusim that is not there: its names are classes that can be derived from, but not made."""
+
+        def __getattr__(self, name):
+            if name.startswith("__"):
+                raise AttributeError(name)
+            made = type(name, (), {"__new__": _refuse})
+            setattr(self, name, made)
+            return made
+
+    accuracy, forces, integrators, simulation, system, units = (_Absent() for _ in range(6))
 
 __all__ = ["accusim", "accuracy", "forces", "integrators", "simulation", "system", "units"]
