@@ -1525,11 +1525,12 @@ int acs_reduce_conserved(const double* pos, const double* vel, const int32_t* sp
 // Some callers cannot allocate device memory when they need forces: code that owns every byte of the GPU
 // through its own pool, real-time loops that forbid allocation after start-up, or plug-in hosts that hand
 // out only input and output buffers. acs_lj_fp64_noalloc serves them: it runs the same FP64 LJ kernel as
-// acs_lj_fp64, but its reduction scratch (one FP64 partial per 256-atom block plus a completion counter)
-// lives in the fixed device array below instead of a caller-provided work buffer.
+// acs_lj_fp64, but its reduction scratch (one FP64 partial per block plus a completion counter) lives in the
+// fixed device array below instead of a caller-provided work buffer, and it gathers from the caller's arrays.
 //
-// The array is 64 KiB + 256 B and exists on every GPU that loads this library until the process exits;
-// it bounds n at kNoAllocMaxAtoms = 2,097,152 atoms. All calls share it, so calls whose work overlaps on the
+// The array is 64 KiB + 256 B and exists on every GPU that loads this library until the process exits; it bounds
+// n at kNoAllocMaxAtoms = 2,097,152 atoms: a block takes 256 atoms, or fewer (down to 8) while the atoms' threads
+// stay within kMostThreads. All calls share it, so calls whose work overlaps on the
 // GPU (different streams, or different host threads on one device) race and corrupt each other's energy;
 // serialise them. The completion counter is cleared at the start of every call; the partials are fully
 // overwritten by each call.
@@ -1537,6 +1538,7 @@ namespace {
 
 constexpr int64_t kNoAllocMaxBlocks = 8192;                   // 8192 partials of 8 bytes = 64 KiB
 constexpr int64_t kNoAllocMaxAtoms = kNoAllocMaxBlocks * kBlock;  // 2,097,152
+static_assert(kMostThreads / kBlock <= kNoAllocMaxBlocks && 2 * kLjThreads <= kMostThreads, "partials of every split");
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocMaxBlocks * 8 + 256];
 
 // The address is looked up once per CUDA context (the primary context of each device, or any context a driver-API

@@ -910,12 +910,14 @@ __device__ __noinline__ bool band_accept(const double* __restrict__ xa, int64_t 
 
 // Rebuild of flagged replicas and per-replica record reduction. Cooperative launch (all blocks resident);
 // each of a rebuild's phases ends in a grid barrier, 2 to 3 us with its first loads, which is what small systems'
-// rebuilds cost: five barriers before the list build with one replica, a sixth for the tile list of several (ten
-// before counts were left clear for the next rebuild, the scan and the in-cell order taken in one phase each: 864-atom
-// argon 36 -> 19 us of a rebuild's phases, 48 replicas 9.3 -> 8.5 ms for 50 steps).
-// every wait is bounded and reports ACS_FLAG_TIMEOUT instead of hanging. EX: the engine has DSF exclusions
+// rebuilds cost: five barriers before the list build with one replica of up to 4096 cells, two more for the scan of one
+// with more, one more for the tile list of several replicas (ten before counts were left clear for the next rebuild, the
+// scan and the in-cell order taken in one phase each: 864-atom argon 36 -> 19 us of a rebuild's phases, 48 replicas
+// 9.3 -> 8.5 ms for 50 steps).
+// Every wait is bounded and reports ACS_FLAG_TIMEOUT instead of hanging. EX: the engine has DSF exclusions
 // (excluded pairs' list entries get the flag E.ex_bit). ATOMS: the lists a warp per atom (engines of 8 and more threads
-// per atom, whose grids leave registers to spare), else a warp per cell.
+// per atom, whose grids leave registers to spare), else a warp per cell, at 80 registers for three blocks an SM, which
+// spills 108 bytes a thread (168 read back).
 template <bool EX, bool ATOMS>
 __global__ void __launch_bounds__(256, ATOMS ? 2 : 3) k_rebuild(Eng E, int dst, int rec, int rec_idx, int force_all) {
   __shared__ unsigned char fl[kMaxRep];

@@ -301,8 +301,9 @@ class Engine:
                    "acs_engine_run_timed")
         return out[0] / max(out[2], 1), out[1] / max(out[3], 1), out[0] + out[1]
 
-    PHASES = {1: "flags", 2: "clear", 3: "bin", 4: "scan_a", 5: "scan_b", 6: "scan_c", 7: "scatter", 8: "sort",
-              9: "gather", 10: "commit", 15: "list_build_block0"}
+    # scan_a and scan_b stay zero where every replica's cells are few chunks (one phase scans them)
+    PHASES = {1: "flags", 3: "bin", 4: "scan_a", 5: "scan_b", 6: "scan_c", 7: "scatter", 9: "gather", 10: "commit",
+              15: "list_build_block0"}
 
     def phase_times(self, clear=True):
         """List-maintenance phase times (ms, accumulated) from the device global timer."""

@@ -18,11 +18,12 @@
 extern "C" {
 #endif
 
-/* 2.5 to 6.1 KB per atom up to 49,152 atoms (phase factors, real-space parts), 1 KB above, and 1 KB per k-vector. */
+/* 1.5 to 6.1 KB per atom up to 49,152 atoms (real-space parts, phase factors), 1 KB above; 1 KB per k-vector; 144 KB. */
 size_t acs_ewald_work_bytes(int64_t n, int32_t K);
 /* pos (n x 3, m), q (n, C), kvec (K x 3, 1/m) and kw (K) are device arrays. force = k * f (N);
- * Any k-vectors are taken; a set of small integer multiples of 2 pi / box edge that holds each vector's mirror image
- * once (the reference's) runs on tabulated phase factors, decided on the device at each call.
+ * Any k-vectors are taken; a set of integer multiples, up to 16 per axis, of 2 pi / box edge that holds each vector's
+ * mirror image once (the reference's up to kmax 16) runs on tabulated phase factors, decided on the device at each call;
+ * any other takes a sine and a cosine per atom and vector.
  * energy3_dev[0] = real-space pair sum (unscaled), [1] = sum_k w_k |S_k|^2 (unscaled): the host forms
  * U = k * (energy3[0] + 2 pi / V * energy3[1] - alpha / sqrt(pi) * sum q^2). */
 int acs_ewald_fp64(const double* pos, const double* q, int64_t n, const double* box3, const double* kvec,
