@@ -810,36 +810,46 @@ struct PairSplit {
 
 // About how many neighbours an atom has in its list (all atoms without one), from the density and the cutoff alone: the
 // split decides the order of an atom's sum, which must not depend on the buffer the caller gave the list (its capacity).
-// A list holds the neighbours to the cutoff plus a skin, 1.4 times those inside in the usual 0.3 of 2.5. Without a box: no
-// statement (infinite).
+// A list holds the neighbours to the cutoff plus a skin, 1.4 times those inside in the usual 0.3 of 2.5. Without a box the
+// density is not known: few, but more than a gas has.
 double pairs_per_atom(int64_t n, bool list, const double* box3, double rc) {
   if (!list) return (double)n;
-  if (!box3) return HUGE_VAL;
+  if (!box3) return std::min((double)n, 24.0);
   const double V = fabs(box3[0] * box3[1] * box3[2]);
   return V > 0.0 ? std::min((double)n, 1.4 * 4.0 / 3.0 * M_PI * rc * rc * rc * ((double)n / V)) : (double)n;
 }
 
-// The fewest phases (at most 32) that give `threads`; then, if `spread`, more while each thread keeps kPhaseEntries
-// of an atom's pairs, up to kMostThreads in all. 151,552 threads are resident, so a split below that leaves places
-// empty, one of a few waves loses its last one, and a thread with few entries is all prologue. DSF terms are long enough
-// to want several waves: 32,768 ions 141 us at 131,072 threads, 118 at 262,144, 112 at 524,288; 175,616 ions 678, 595,
-// 544; 64,000 ions 224, 213, 205 (209 at 1,048,576). LJ with 79 entries an atom does not: 32,000 atoms 18.5 us at
-// 128,000 threads, 21.6 at 256,000, 21.5 at 64,000; 55,296 atoms 25.5 at 110,592, 28.0 at 221,184, 35.0 at 55,296;
-// 1,048,576 atoms 0.355 ms with one phase, 0.372 with two, 0.430 with four. With 351 entries it does: 110,592 ions
-// 135 us with four phases, 157 with two, 147 with eight; 175,616 ions 210 with four, 300 with one.
-constexpr int64_t kMostThreads = 1 << 20, kLjThreads = 98304, kDsfThreads = 524288;
-constexpr double kPhaseEntries = 56.0;
-PairSplit pair_split(int64_t n, int64_t threads, double pairs, bool spread) {
+// The fewest phases (at most 32) that give kHalfFilled threads; then more, up to `threads` and kMostThreads in all, while
+// each thread keeps `entries` of an atom's pairs. 151,552 threads are resident: half of them hide the latency of a call
+// with few pairs, and more only add blocks whose sums meet at the end (LJ gas, 0.3 entries an atom: 12,000 atoms 11.3 us
+// with 96,000 threads, 13.6 with 192,000). A thread with few entries is all prologue. DSF terms are long enough to want
+// several waves, if there are pairs: 32,768 ions with 351 entries 141 us at 131,072 threads, 118 at 262,144, 112 at
+// 524,288; 175,616 ions 678, 595, 544; 64,000 with 78 entries 83, 72, 72 us at 128,000, 256,000 and 512,000; with 22
+// entries 33, 31, 35; with 0.3 entries 12, 15, 21 (a thread per atom, as it was before the split: 17). LJ with 79 entries
+// an atom does not: 32,000 atoms 18.5 us at 128,000 threads, 21.6 at 256,000, 21.5 at 64,000; 12,000 atoms 17.7 at 96,000,
+// 19.7 at 192,000; 55,296 atoms 25.5 at 110,592, 28.0 at 221,184, 35.0 at 55,296; 1,048,576 atoms 0.355 ms with one
+// phase, 0.372 with two, 0.430 with four. With 351 entries it does: 110,592 ions 135 us with four phases, 157 with two,
+// 147 with eight; 175,616 ions 210 with four, 300 with one.
+constexpr int64_t kMostThreads = 1 << 20, kHalfFilled = 75776, kDsfThreads = 524288;
+constexpr double kLjEntries = 56.0, kDsfEntries = 8.0;
+PairSplit pair_split(int64_t n, double pairs, int64_t threads, double entries) {
   PairSplit s;
   s.log2_phases = 0;
-  while (s.log2_phases < 5 && (n << s.log2_phases) < threads) ++s.log2_phases;
-  while (spread && pairs < HUGE_VAL && s.log2_phases < 5 && (n << (s.log2_phases + 1)) <= kMostThreads &&
-         pairs >= kPhaseEntries * (2 << s.log2_phases))
+  while (s.log2_phases < 5 && (n << s.log2_phases) < kHalfFilled) ++s.log2_phases;
+  while (s.log2_phases < 5 && (n << s.log2_phases) < threads && (n << (s.log2_phases + 1)) <= kMostThreads &&
+         pairs >= entries * (2 << s.log2_phases))
     ++s.log2_phases;
   s.atoms = kBlock >> s.log2_phases;
   s.blocks = ceil_div(n, s.atoms);
   return s;
 }
+
+// Whether the gathers are worth a launch that packs the atoms first. In small systems, and in larger ones with few pairs, it
+// costs more than it gives: 400 atoms 11.0 us packed, 9.5 from the caller's arrays, at any density; 4000 atoms with 78
+// entries 13.5, 12.7 (with 345 entries 19.8, 18.9); 12,000 with 33 entries 13.5, 12.7, with 78 17.6, 17.0, with 344 36.1,
+// 40.5; 26,000 with 0.3 entries 11.2, 9.9, with 78 21.9, 24.9; DSF at the same sizes 10.0, 8.6; 15.6, 14.6 (30.2, 29.9);
+// 17.6, 16.6, 25.9, 24.8, 60.7, 63.7; 10.9, 9.4, 38.7, 40.1. The same results bit for bit.
+bool pack_gathers(int64_t n, double pairs) { return n >= 32768 || (n >= 6000 && (double)n * pairs >= 1e6); }
 
 // Sums the phases' values of every atom of the block in phase order; the result is in phase 0's threads.
 __device__ __forceinline__ void sum_phases(const PairSplit& sp, double (&v)[4]) {
@@ -859,8 +869,8 @@ __device__ __forceinline__ void sum_phases(const PairSplit& sp, double (&v)[4]) 
 // cycle, 0.29 ms for 82M entries, and the kernel takes 0.30 (one thread per atom over the caller's arrays, with branches
 // around each pair and three rounding instructions per minimum image: 0.67). Three gathers and the next list entries
 // in flight at 64 registers; more of either loses the occupancy that hides the FP64 chains (0.32 to 0.44 measured). An
-// 864-atom box: 52 -> 5.8 us; 256 atoms without a list: 92 -> 6.8. PACKED gathers one 256-bit record per neighbour, otherwise from the caller's arrays (the
-// entry point without a work buffer). ONE: a single species, its constants in registers; else the species-pair tables
+// 864-atom box: 52 -> 5.8 us; 256 atoms without a list: 92 -> 6.8. PACKED gathers one 256-bit record per neighbour,
+// otherwise from the caller's arrays (pack_gathers; the entry point without a work buffer). ONE: a single species, its constants in registers; else the species-pair tables
 // are staged in shared memory (a kernel parameter indexed per thread serialises).
 template <bool DENSE, bool PACKED, bool ONE>
 __global__ void __launch_bounds__(kBlock, 4) k_lj64(const double* __restrict__ pos, const int32_t* __restrict__ sp,
@@ -998,12 +1008,12 @@ void launch_lj64(const double* pos, const int32_t* sp, const Packed* pk, int64_t
                                                                    force, partials, ticket, energy);
 }
 
-PairSplit lj_split(int64_t n, bool list, const double* box3, int n_species, const double* eps_tab, const double* sig_tab,
-                   double cutoff) {
+double lj_pairs_per_atom(int64_t n, bool list, const double* box3, int n_species, const double* eps_tab,
+                         const double* sig_tab, double cutoff) {
   double sig = 0.0;   // the largest of a pair that interacts
   for (int a = 0; a < n_species * n_species; ++a)
     if (eps_tab[a] > 0.0) sig = std::max(sig, sig_tab[a]);
-  return pair_split(n, kLjThreads, pairs_per_atom(n, list, box3, cutoff * sig), true);
+  return pairs_per_atom(n, list, box3, cutoff * sig);
 }
 
 LJTab lj_tables(int n_species, const double* eps_tab, const double* sig_tab, double cutoff) {
@@ -1021,13 +1031,14 @@ LJTab lj_tables(int n_species, const double* eps_tab, const double* sig_tab, dou
   return t;
 }
 
-// DSF forces and energy, FP64, over packed positions and charges, the gather and the list entry after it in flight. Bound
+// DSF forces and energy, FP64, the gather and the list entry after it in flight (PACKED as for k_lj64). Bound
 // by FP64 issue: about 90 FP64 operations per list entry (two thirds of the entries lie inside the cutoff, but nearly
 // every warp holds one that does), half the pipe's rate on 64,000 ions. 4096 ions (351 list entries each): 430 us with
 // one thread per atom, sqrt, erfc, exp and two divisions a pair, 34 with the split, 28 with erfc_exp; 64,000 ions:
 // 640, 301 and 229.
-template <bool DENSE>
-__global__ void __launch_bounds__(kBlock, 4) k_dsf64(const Packed* __restrict__ pk, int64_t n, ImageBox box,
+template <bool DENSE, bool PACKED>
+__global__ void __launch_bounds__(kBlock, 4) k_dsf64(const double* __restrict__ pos, const double* __restrict__ q,
+                                                      const Packed* __restrict__ pk, int64_t n, ImageBox box,
                                                       const int32_t* __restrict__ nbr, const int32_t* __restrict__ nnb,
                                                       int maxnb, const int32_t* __restrict__ ex_start,
                                                       const int32_t* __restrict__ ex_idx, DSFPar P, PairSplit split,
@@ -1039,7 +1050,16 @@ __global__ void __launch_bounds__(kBlock, 4) k_dsf64(const Packed* __restrict__ 
   double v[4] = {0.0, 0.0, 0.0, 0.0};
   double qi = 0.0;
   if (i < n) {
-    const Packed me = ld_packed(pk + i);
+    auto gather = [&](int64_t j) {
+      if (PACKED) return ld_packed(pk + j);
+      Packed o;
+      o.x = pos[3 * j];
+      o.y = pos[3 * j + 1];
+      o.z = pos[3 * j + 2];
+      o.w = q[j];
+      return o;
+    };
+    const Packed me = gather(i);
     qi = me.w;
     const int xs = ex_start ? ex_start[i] : 0, xe = ex_start ? ex_start[i + 1] : 0;
     const int32_t* __restrict__ row = DENSE ? nullptr : nbr + nbr_slot(i, 0, maxnb);
@@ -1049,7 +1069,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_dsf64(const Packed* __restrict__ 
     int32_t jn = entry(phase);
     for (int64_t k = phase; k < m; k += phases) {
       const int32_t j = jn;
-      const Packed o = ld_packed(pk + j);
+      const Packed o = gather(j);
       jn = entry(k + phases);
       double dx = sub(o.x, me.x), dy = sub(o.y, me.y), dz = sub(o.z, me.z);
       if (!near_image(dx, dy, dz, box)) image3(dx, dy, dz, box);
@@ -1390,14 +1410,17 @@ size_t acs_force_work_bytes(int64_t n) {
   return align256(force_blocks(n) * 8) + 256 + align256((size_t)std::max<int64_t>(n, 1) * sizeof(Packed)) + 256;
 }
 
-// Carves a force call's work buffer and launches the packing kernel, which also clears the ticket.
+// Carves a force call's work buffer and clears the ticket; with `packed`, by the packing kernel, which it launches.
 static int force_setup(const double* pos, const int32_t* sp, const double* q, int64_t n, void* work, size_t work_bytes,
-                       double** partials, unsigned int** ticket, Packed** pk, cudaStream_t s) {
+                       const PairSplit& split, bool packed, double** partials, unsigned int** ticket, Packed** pk,
+                       cudaStream_t s) {
   if (work_bytes < acs_force_work_bytes(n) || !work) return ACS_ERR_WORKSPACE;
   char* w = (char*)(((uintptr_t)work + 255) & ~(uintptr_t)255);
   *partials = (double*)w; w += align256(force_blocks(n) * 8);
   *ticket = (unsigned int*)w; w += 256;
   *pk = (Packed*)w;
+  if (!packed)   // one block adds up without the ticket
+    return split.blocks == 1 || cudaMemsetAsync(*ticket, 0, 4, s) == cudaSuccess ? ACS_OK : ACS_ERR_CUDA;
   k_pack<<<(int)ceil_div(n, kBlock), kBlock, 0, s>>>(pos, sp, q, n, *pk, *ticket);
   return launch_status();
 }
@@ -1421,15 +1444,16 @@ int acs_lj_fp64(const double* pos, const int32_t* sp, int64_t n, const double* b
   double* partials;
   unsigned int* ticket;
   Packed* pk;
-  int st = force_setup(pos, sp, nullptr, n, work, work_bytes, &partials, &ticket, &pk, s);
+  const double pairs = lj_pairs_per_atom(n, nbr, box3, n_species, eps_tab, sig_tab, cutoff);
+  const PairSplit split = pair_split(n, pairs, kMostThreads, kLjEntries);
+  const bool packed = pack_gathers(n, pairs);
+  int st = force_setup(pos, sp, nullptr, n, work, work_bytes, split, packed, &partials, &ticket, &pk, s);
   if (st) return st;
   const LJTab t = lj_tables(n_species, eps_tab, sig_tab, cutoff);
-  const PairSplit split = lj_split(n, nbr, box3, n_species, eps_tab, sig_tab, cutoff);
   const ImageBox b = image_box(box3, periodic);
-  if (n_species == 1)
-    launch_lj64<true, true>(pos, sp, pk, n, b, nbr, nnb, maxnb, t, split, force, partials, ticket, energy_dev, s);
-  else
-    launch_lj64<true, false>(pos, sp, pk, n, b, nbr, nnb, maxnb, t, split, force, partials, ticket, energy_dev, s);
+  auto launch = n_species == 1 ? (packed ? launch_lj64<true, true> : launch_lj64<false, true>)
+                               : (packed ? launch_lj64<true, false> : launch_lj64<false, false>);
+  launch(pos, sp, pk, n, b, nbr, nnb, maxnb, t, split, force, partials, ticket, energy_dev, s);
   return launch_status();
 }
 
@@ -1444,7 +1468,10 @@ int acs_dsf_fp64(const double* pos, const double* q, int64_t n, const double* bo
   double* partials;
   unsigned int* ticket;
   Packed* pk;
-  int st = force_setup(pos, nullptr, q, n, work, work_bytes, &partials, &ticket, &pk, s);
+  const double pairs = pairs_per_atom(n, nbr, box3, rcut);
+  const PairSplit split = pair_split(n, pairs, kDsfThreads, kDsfEntries);
+  const bool packed = pack_gathers(n, pairs);
+  int st = force_setup(pos, nullptr, q, n, work, work_bytes, split, packed, &partials, &ticket, &pk, s);
   if (st) return st;
   DSFPar P;
   P.a = alpha;
@@ -1457,13 +1484,10 @@ int acs_dsf_fp64(const double* pos, const double* q, int64_t n, const double* bo
   P.fshift = P.erc / (rcut * rcut) + P.c * exp(-((alpha * rcut) * (alpha * rcut))) / rcut;
   P.self_coef = P.erc / (2.0 * rcut) + alpha / sqrt(M_PI);
   const ImageBox b = image_box(box3, periodic);
-  const PairSplit split = pair_split(n, kDsfThreads, pairs_per_atom(n, nbr, box3, rcut), false);
-  if (nbr)
-    k_dsf64<false><<<(int)split.blocks, kBlock, 0, s>>>(pk, n, b, nbr, nnb, maxnb, ex_start, ex_idx, P, split, force,
-                                                       partials, ticket, energy_dev);
-  else
-    k_dsf64<true><<<(int)split.blocks, kBlock, 0, s>>>(pk, n, b, nullptr, nullptr, 0, ex_start, ex_idx, P, split, force,
-                                                      partials, ticket, energy_dev);
+  auto kernel = nbr ? (packed ? k_dsf64<false, true> : k_dsf64<false, false>)
+                    : (packed ? k_dsf64<true, true> : k_dsf64<true, false>);
+  kernel<<<(int)split.blocks, kBlock, 0, s>>>(pos, q, pk, n, b, nbr, nnb, maxnb, ex_start, ex_idx, P, split, force, partials,
+                                              ticket, energy_dev);
   return launch_status();
 }
 
@@ -1526,7 +1550,7 @@ int acs_reduce_conserved(const double* pos, const double* vel, const int32_t* sp
 // through its own pool, real-time loops that forbid allocation after start-up, or plug-in hosts that hand
 // out only input and output buffers. acs_lj_fp64_noalloc serves them: it runs the same FP64 LJ kernel as
 // acs_lj_fp64, but its reduction scratch (one FP64 partial per block plus a completion counter) lives in the
-// fixed device array below instead of a caller-provided work buffer, and it gathers from the caller's arrays.
+// fixed device array below instead of a caller-provided work buffer, and it always gathers from the caller's arrays.
 //
 // The array is 64 KiB + 256 B and exists on every GPU that loads this library until the process exits; it bounds
 // n at kNoAllocMaxAtoms = 2,097,152 atoms: a block takes 256 atoms, or fewer (down to 8) while the atoms' threads
@@ -1538,7 +1562,7 @@ namespace {
 
 constexpr int64_t kNoAllocMaxBlocks = 8192;                   // 8192 partials of 8 bytes = 64 KiB
 constexpr int64_t kNoAllocMaxAtoms = kNoAllocMaxBlocks * kBlock;  // 2,097,152
-static_assert(kMostThreads / kBlock <= kNoAllocMaxBlocks && 2 * kLjThreads <= kMostThreads, "partials of every split");
+static_assert(kMostThreads / kBlock <= kNoAllocMaxBlocks && 2 * kHalfFilled <= kMostThreads, "partials of every split");
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocMaxBlocks * 8 + 256];
 
 // The address is looked up once per CUDA context (the primary context of each device, or any context a driver-API
@@ -1611,7 +1635,8 @@ extern "C" int acs_lj_fp64_noalloc(const double* pos, const int32_t* sp, int64_t
   unsigned int* ticket = (unsigned int*)((char*)scratch + kNoAllocMaxBlocks * 8);
   if (cudaMemsetAsync(ticket, 0, 4, s) != cudaSuccess) return ACS_ERR_CUDA;
   const LJTab t = lj_tables(n_species, eps_tab, sig_tab, cutoff);
-  const PairSplit split = lj_split(n, nbr, box3, n_species, eps_tab, sig_tab, cutoff);
+  const PairSplit split =
+      pair_split(n, lj_pairs_per_atom(n, nbr, box3, n_species, eps_tab, sig_tab, cutoff), kMostThreads, kLjEntries);
   const ImageBox b = image_box(box3, periodic);
   if (n_species == 1)   // the same arithmetic as acs_lj_fp64, bit for bit
     launch_lj64<false, true>(pos, sp, nullptr, n, b, nbr, nnb, maxnb, t, split, force, partials, ticket, energy_dev, s);
