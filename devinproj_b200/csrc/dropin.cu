@@ -743,26 +743,30 @@ __global__ void k_pairs(const int32_t* __restrict__ nbr, const int32_t* __restri
   }
 }
 
-__device__ __forceinline__ bool moved(const double* __restrict__ pos, const double* __restrict__ pos0, int64_t i,
-                                      const ImageBox& box, double half_skin2) {
-  double dx = sub(pos[3 * i], pos0[3 * i]), dy = sub(pos[3 * i + 1], pos0[3 * i + 1]),
-         dz = sub(pos[3 * i + 2], pos0[3 * i + 2]);
+__device__ __forceinline__ bool moved(double dx, double dy, double dz, const ImageBox& box, double half_skin2) {
   image3(dx, dy, dz, box);
   return !(norm2(dx, dy, dz) < half_skin2);   // NaN also forces a rebuild, as in the reference
 }
 
 // One block's answer for up to kMovedAtoms atoms, without the clear that the grid's needs before it: a small system's
-// skin test is launches (a clear and a kernel, 3 us, for 2 us of one kernel).
+// skin test is launches. The loads of a thread's atoms go out together (4096 atoms:
+// 5.9 us one after the other, 5.3 so; 3.1 on the grid, and the clear).
 constexpr int kMovedAtoms = 4096;
 __global__ void __launch_bounds__(1024) k_displacement_block(const double* __restrict__ pos,
                                                              const double* __restrict__ pos0, int n, ImageBox box,
                                                              double half_skin2, int32_t* flag) {
+  constexpr int kA = kMovedAtoms / 1024;
+  double d[kA][3];
+#pragma unroll
+  for (int q = 0; q < kA; ++q) {
+    const int i = threadIdx.x + 1024 * q;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) d[q][c] = i < n ? sub(pos[3 * i + c], pos0[3 * i + c]) : 0.0;
+  }
   bool any = false;
 #pragma unroll
-  for (int q = 0; q < kMovedAtoms / 1024; ++q) {
-    const int i = threadIdx.x + 1024 * q;
-    if (i < n) any = any || moved(pos, pos0, i, box, half_skin2);
-  }
+  for (int q = 0; q < kA; ++q)
+    if ((int)threadIdx.x + 1024 * q < n) any = any || moved(d[q][0], d[q][1], d[q][2], box, half_skin2);
   const int r = __syncthreads_or(any);
   if (threadIdx.x == 0) *flag = r ? 1 : 0;
 }
@@ -770,7 +774,9 @@ __global__ void __launch_bounds__(1024) k_displacement_block(const double* __res
 __global__ void k_displacement(const double* __restrict__ pos, const double* __restrict__ pos0, int64_t n, ImageBox box,
                                double half_skin2, int32_t* flag) {
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n && moved(pos, pos0, i, box, half_skin2)) *flag = 1;
+  if (i < n && moved(sub(pos[3 * i], pos0[3 * i]), sub(pos[3 * i + 1], pos0[3 * i + 1]), sub(pos[3 * i + 2], pos0[3 * i + 2]),
+                     box, half_skin2))
+    *flag = 1;
 }
 
 // ------------------------------------------------------------------------------------ forces --
@@ -1118,7 +1124,7 @@ __device__ __forceinline__ double py_mod(double x, double L) {
   return r;
 }
 
-// Calls f(element, atom, axis) for the 768 components of each block's 256 atoms, three per thread, 256 apart: the arrays
+// Calls f(element, atom, axis, q) for the 768 components of each block's 256 atoms, three per thread, 256 apart: the arrays
 // stream, where an atom per thread reads and writes 24-byte strides.
 template <class F>
 __device__ __forceinline__ void for_components(int64_t n, F&& f) {
@@ -1127,15 +1133,22 @@ __device__ __forceinline__ void for_components(int64_t n, F&& f) {
 #pragma unroll
   for (int q = 0; q < 3; ++q) {
     const int l = threadIdx.x + kBlock * q;
-    if (l < m) f(3 * i0 + l, i0 + l / 3, l % 3);
+    if (l < m) f(3 * i0 + l, i0 + l / 3, l % 3, q);
   }
 }
 
 // pos += dt vel, pos %= L. In (0, L) the remainder is x itself, in (L, 2L) and (-L, 0) one exact or IEEE subtraction or
-// addition, as py_mod's fmod has it; its loop is left to the others. 1M atoms 22 -> 12 us (its bytes take 11.5).
+// addition, as py_mod's fmod has it; its loop is left to the others. A thread's
+// loads go out together: with each store before the next component's load a small system took 4.4 us, an atom per thread
+// 3.1, and so 3.2; 1M atoms 19 us an atom per thread, 10.1, and 8.3 (L2 holds part of it; its bytes take 11.5 from HBM).
 __global__ void k_drift_wrap(double* __restrict__ pos, const double* __restrict__ vel, int64_t n, double dt, ImageBox box) {
-  for_components(n, [&](int64_t e, int64_t, int d) {
-    double x = add(pos[e], mul(dt, vel[e]));
+  double p[3], v[3];
+  for_components(n, [&](int64_t e, int64_t, int, int q) {
+    p[q] = pos[e];
+    v[q] = vel[e];
+  });
+  for_components(n, [&](int64_t e, int64_t, int d, int q) {
+    double x = add(p[q], mul(dt, v[q]));
     if (box.periodic) {
       const double L = d == 0 ? box.L[0] : d == 1 ? box.L[1] : box.L[2];
       if (!(x > 0.0 && x < L)) x = x > L && x < 2.0 * L ? sub(x, L) : (x < 0.0 && x > -L ? add(x, L) : py_mod(x, L));
@@ -1157,7 +1170,7 @@ struct MassTab {
 
 __global__ void k_accel(double* __restrict__ acc, const double* __restrict__ force, const int32_t* __restrict__ sp,
                         const __grid_constant__ MassTab mt, int64_t n) {
-  for_components(n, [&](int64_t e, int64_t i, int) { acc[e] = div(force[e], mt.m[sp[i]]); });   // 1M atoms 20 -> 11 us
+  for_components(n, [&](int64_t e, int64_t i, int, int) { acc[e] = div(force[e], mt.m[sp[i]]); });   // 1M atoms 20 -> 11 us
 }
 
 __global__ void __launch_bounds__(kBlock) k_conserved(const double* __restrict__ pos, const double* __restrict__ vel,
