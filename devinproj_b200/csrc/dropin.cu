@@ -749,8 +749,8 @@ __device__ __forceinline__ bool moved(double dx, double dy, double dz, const Ima
 }
 
 // One block's answer for up to kMovedAtoms atoms, without the clear that the grid's needs before it: a small system's
-// skin test is launches. The loads of a thread's atoms go out together (4096 atoms:
-// 5.9 us one after the other, 5.3 so; 3.1 on the grid, and the clear).
+// skin test is launches. The loads of a thread's atoms go out together (4096 atoms: 5.9 us one after the other, 5.3 so; the
+// grid's kernel takes 3.1, and the clear).
 constexpr int kMovedAtoms = 4096;
 __global__ void __launch_bounds__(1024) k_displacement_block(const double* __restrict__ pos,
                                                              const double* __restrict__ pos0, int n, ImageBox box,
@@ -1138,9 +1138,9 @@ __device__ __forceinline__ void for_components(int64_t n, F&& f) {
 }
 
 // pos += dt vel, pos %= L. In (0, L) the remainder is x itself, in (L, 2L) and (-L, 0) one exact or IEEE subtraction or
-// addition, as py_mod's fmod has it; its loop is left to the others. A thread's
-// loads go out together: with each store before the next component's load a small system took 4.4 us, an atom per thread
-// 3.1, and so 3.2; 1M atoms 19 us an atom per thread, 10.1, and 8.3 (L2 holds part of it; its bytes take 11.5 from HBM).
+// addition, as py_mod's fmod has it; its loop is left to the others. A thread's loads
+// go out together: a small system takes 3.2 us so, 4.4 with each store before the next component's load, 3.1 with an atom
+// per thread; 1M atoms 8.3, 10.1 and 19 us (L2 holds part of them; from HBM the bytes take 11.5).
 __global__ void k_drift_wrap(double* __restrict__ pos, const double* __restrict__ vel, int64_t n, double dt, ImageBox box) {
   double p[3], v[3];
   for_components(n, [&](int64_t e, int64_t, int, int q) {

@@ -798,11 +798,15 @@ __device__ __noinline__ int band_code(const Eng& E, const RepDev& R, int64_t i, 
 // The list of atom i built by one warp: a ballot over 32 candidates keeps the accepted ones in stencil order and
 // ascending slot. The 27 stencil cells' slot ranges are read by 27 lanes at once and the candidates run through them as
 // one packed sequence, 32 kU loads in flight: a warp that walked cell after cell, each behind dependent loads from L2,
-// spent a small system's build waiting (864-atom argon 14.4 us of list build per rebuild, 10.4 now; 4096-ion NaCl, 27
-// cells of 152 ions, 94 us, 81 now). `shift`: 27 entries of shared memory for the image shifts, one per stencil cell.
+// spent a small system's build waiting. A candidate finds its cell among the occupied ones from a bit mask of where they
+// begin, as in the build per cell; a binary search by shuffles, 12 of them per 32 candidates, cost as much as the rest of
+// the screen. A whole rebuild with its loads (set_state), cell after cell, by search and by mask: 864 LJ atoms 79, 59, 52
+// us; 4096 atoms with 345 entries 186, 137, 116; 16,384 of them 341, 337, 269; 64,000 LJ atoms in cells three list radii
+// wide 3.17, 4.05, 3.06 ms; 700 replicas of 256 atoms in one cell each 464, 513, 463 us. `cells`: 27 entries of shared
+// memory for the occupied cells in order: this atom less the image shift, and entry (slot | code) minus position.
 template <bool EX, int kU>
 __device__ __forceinline__ void list_atom_warp(const Eng& E, const RepDev& R, int64_t i, int dst, int lane,
-                                               float4* shift) {
+                                               float4* cells) {
   const float4* __restrict__ im = E.img[dst];
   const float4 pi = im[i];
   const float rl2f = (float)R.rl2, lo_f = rl2f * (1.0f - 1e-4f), hi_f = rl2f * (1.0f + 1e-4f);
@@ -810,56 +814,67 @@ __device__ __forceinline__ void list_atom_warp(const Eng& E, const RepDev& R, in
   const float L0 = (float)R.L[0], L1 = (float)R.L[1], L2 = (float)R.L[2];
   // lane st = 9 (a + 1) + 3 (b + 1) + (d + 1): its stencil cell's first slot, length and place P in the sequence
   int sk0 = 0, slen = 0;
-  if (lane < 27) {
-    const int a = lane / 9 - 1, b = (lane / 3) % 3 - 1, d = lane % 3 - 1;
-    if ((!one0 || a == 0) && (!one1 || b == 0) && (!one2 || d == 0)) {
-      int c0, c1, c2;
-      cell_coords(E.cellid[i] - R.cellbase, R, c0, c1, c2);
-      const int n0 = wrapc(c0 + a, R.nc[0]), n1 = wrapc(c1 + b, R.nc[1]), n2 = wrapc(c2 + d, R.nc[2]);
-      const int p = E.crank[R.cellbase + (n0 * R.nc[1] + n1) * R.nc[2] + n2];
-      sk0 = E.start[p];
-      slen = E.start[p + 1] - sk0;
+  const int a = lane / 9 - 1, b = (lane / 3) % 3 - 1, d = lane % 3 - 1;
+  if (lane < 27 && (!one0 || a == 0) && (!one1 || b == 0) && (!one2 || d == 0)) {
+    int c0, c1, c2;
+    cell_coords(E.cellid[i] - R.cellbase, R, c0, c1, c2);
+    const int n0 = wrapc(c0 + a, R.nc[0]), n1 = wrapc(c1 + b, R.nc[1]), n2 = wrapc(c2 + d, R.nc[2]);
+    const int p = E.crank[R.cellbase + (n0 * R.nc[1] + n1) * R.nc[2] + n2];
+    sk0 = E.start[p];
+    slen = E.start[p + 1] - sk0;
+  }
+  // small replicas that are one cell (kU 1: beside the build per cell, for which their atoms are units) need no search
+  const bool lone = kU == 1 && one0 && one1 && one2;
+  int P = 0, T;
+  if (lone) {
+    T = __shfl_sync(0xffffffffu, slen, 13);
+  } else {
+    int incl = slen;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += y;
     }
-    // the shift taken off this atom, and the entry's code
-    shift[lane] = make_float4(pi.x - a * R.csf[0], pi.y - b * R.csf[1], pi.z - d * R.csf[2],
-                              __int_as_float((a + 1) + 3 * (b + 1) + 9 * (d + 1)));
+    P = incl - slen;
+    T = __shfl_sync(0xffffffffu, incl, 26);
+  }
+  const unsigned below = (1u << lane) - 1u;
+  const unsigned occupied = __ballot_sync(0xffffffffu, slen > 0);
+  if (slen > 0) {
+    const uint32_t entry = (uint32_t)(sk0 - P) + ((uint32_t)((a + 1) + 3 * (b + 1) + 9 * (d + 1)) << kIdxBits);
+    cells[__popc(occupied & below)] =
+        make_float4(pi.x - a * R.csf[0], pi.y - b * R.csf[1], pi.z - d * R.csf[2], __uint_as_float(entry));
   }
   __syncwarp();
-  int incl = slen;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const int y = __shfl_up_sync(0xffffffffu, incl, o);
-    if (lane >= o) incl += y;
-  }
-  const int P = incl - slen, T = __shfl_sync(0xffffffffu, incl, 26);
-  const unsigned below = (1u << lane) - 1u;
+  int rank0 = -1;   // occupied cells begun before the chunk, less one
   int32_t* __restrict__ lst = E.nbr + (i / E.G) * (int64_t)E.maxnb * E.G + (i % E.G);
   int cnt = 0;
   for (int pb = 0; pb < T; pb += 32 * kU) {
-    int k[kU], st[kU];
+    int rank[kU];
+    uint32_t entry[kU];
     float4 pj[kU];
 #pragma unroll
     for (int u = 0; u < kU; ++u) {
       const int p = pb + 32 * u + lane;
-      const int pp = min(p, T - 1);
-      st[u] = 0;   // last stencil cell with P <= pp
-#pragma unroll
-      for (int step = 16; step > 0; step >>= 1) {
-        const int c = st[u] + step;
-        const int Pc = __shfl_sync(0xffffffffu, P, c < 27 ? c : 26);
-        if (c < 27 && Pc <= pp) st[u] = c;
+      rank[u] = 0;
+      if (!lone) {
+        const unsigned off = (unsigned)(P - (pb + 32 * u));
+        const unsigned begins = __reduce_or_sync(0xffffffffu, slen > 0 && off < 32u ? 1u << off : 0u);
+        rank[u] = rank0 + __popc(begins & (below << 1 | 1u));
+        rank0 += __popc(begins);
       }
-      k[u] = __shfl_sync(0xffffffffu, sk0, st[u]) + (pp - __shfl_sync(0xffffffffu, P, st[u]));
+      entry[u] = __float_as_uint(cells[rank[u]].w) + (uint32_t)p;
       pj[u] = make_float4(3e30f, 3e30f, 3e30f, 0.f);   // past the end: r^2 overflows
-      if (p < T) pj[u] = im[k[u]];
+      if (p < T) pj[u] = im[entry[u] & kIdxMask];
     }
 #pragma unroll
     for (int u = 0; u < kU; ++u) {
       if (pb + 32 * u >= T) break;
-      const float4 m = shift[st[u]];
+      const float4 m = cells[rank[u]];
       float x = pj[u].x - m.x, y = pj[u].y - m.y, z = pj[u].z - m.z;
-      int code = __float_as_int(m.w);
-      const bool live = pb + 32 * u + lane < T && k[u] != i;
+      const int k = (int)(entry[u] & kIdxMask), cell = (int)(entry[u] >> kIdxBits);
+      int code = cell;
+      const bool live = pb + 32 * u + lane < T && k != i;
       if (any_one && live) {   // the image of a one-cell axis is found per pair
         if (one0) { const int w = x > 0.5f * L0 ? 1 : (x < -0.5f * L0 ? -1 : 0); x -= w * L0; code -= w; }
         if (one1) { const int w = y > 0.5f * L1 ? 1 : (y < -0.5f * L1 ? -1 : 0); y -= w * L1; code -= 3 * w; }
@@ -870,15 +885,15 @@ __device__ __forceinline__ void list_atom_warp(const Eng& E, const RepDev& R, in
       const bool band = live && q > lo_f && q < hi_f;
       if (__any_sync(0xffffffffu, band)) {
         if (band) {
-          code = band_code(E, R, i, k[u], st[u] / 9 - 1, (st[u] / 3) % 3 - 1, st[u] % 3 - 1);
+          code = band_code(E, R, i, k, cell % 3 - 1, (cell / 3) % 3 - 1, cell / 9 - 1);
           in = code >= 0;
         }
       }
       const unsigned bal = __ballot_sync(0xffffffffu, in);
       const int pos = cnt + __popc(bal & below);
       if (in && pos < E.maxnb) {
-        uint32_t v = (uint32_t)k[u] | ((uint32_t)code << kIdxBits);
-        if (EX && dsf_excluded(E, E.id[i], E.id[k[u]])) v |= E.ex_bit;
+        uint32_t v = (uint32_t)k | ((uint32_t)code << kIdxBits);
+        if (EX && dsf_excluded(E, E.id[i], E.id[k])) v |= E.ex_bit;
         lst[(int64_t)pos * E.G] = (int32_t)v;
       }
       cnt += __popc(bal);
@@ -891,7 +906,7 @@ __device__ __forceinline__ void list_atom_warp(const Eng& E, const RepDev& R, in
       atomicMax(&E.status->need_nbr, cnt);
     }
   }
-  __syncwarp();   // before the next atom's shifts
+  __syncwarp();   // before the next atom's table
 }
 
 // Exact decision for a candidate in the FP32 band around the list radius, on a replica with >= 3 cells per
