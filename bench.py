@@ -57,6 +57,90 @@ def workload(name, seed=0):
     return s, forces, dt, cfg
 
 
+class PlainFluid:
+    """What the LJ workloads need of an accusim `System`, for where accusim cannot be imported: argon on an fcc lattice in a
+    cubic periodic box, with velocities at the workload's temperature."""
+    dim, periodic = 3, True
+
+    def __init__(self, n_cells, seed=0, rho_star=0.8442, T=0.72 * 120.0, L=None):
+        import numpy as np
+        from types import SimpleNamespace
+
+        from devinproj_b200 import configs
+        n = 4 * n_cells ** 3
+        L = (n / rho_star) ** (1 / 3) * configs.AR_SIGMA if L is None else L
+        self.species = [SimpleNamespace(name="Ar", mass=configs.AR_MASS, charge=0.0)]
+        self.box, self.n = np.full(3, L), n
+        self.pos = configs.fcc_positions(n_cells, L)
+        self.sp, self.ids = np.zeros(n, dtype=int), np.arange(n)
+        v = np.random.default_rng(seed).normal(size=(n, 3)) * math.sqrt(configs.k_B * T / configs.AR_MASS)
+        self.vel = v - v.mean(axis=0)
+
+    def copy(self):
+        import copy
+        return copy.deepcopy(self)
+
+
+class PlainLJ:
+    """The workloads' LennardJones there: FP64 forces of a PlainFluid by the C ABI."""
+    cutoff, skin = 2.5, 0.3
+
+    def compute(self, s):
+        import numpy as np
+        import torch
+
+        from devinproj_b200 import _lib, configs
+        from devinproj_b200.device import stream_handle, to_dev
+        from devinproj_b200.forces import DeviceNeighborList
+        pos, sp = to_dev(s.pos), to_dev(s.sp, torch.int32)
+        nl = DeviceNeighborList().build(s, pos, self.cutoff * configs.AR_SIGMA)
+        L = _lib.lib()
+        F, U = torch.empty_like(pos), torch.empty(1, dtype=torch.float64, device="cuda")
+        work = torch.empty(L.acs_force_work_bytes(s.n), dtype=torch.uint8, device="cuda")
+        eps, sig, box = np.array([configs.AR_EPS]), np.array([configs.AR_SIGMA]), np.ascontiguousarray(s.box)
+        _lib.check(L.acs_lj_fp64(pos.data_ptr(), sp.data_ptr(), s.n, box.ctypes.data, 1, nl.nbr.data_ptr(), nl.nnb.data_ptr(),
+                                 nl.maxnb, 1, eps.ctypes.data, sig.ctypes.data, self.cutoff, F.data_ptr(), U.data_ptr(),
+                                 work.data_ptr(), work.numel(), stream_handle()), "acs_lj_fp64")
+        return F.cpu().numpy(), float(U.item())
+
+
+def plain_workload(name, seed=0):
+    """`workload` where accusim cannot be imported (the LJ workloads)."""
+    from devinproj_b200 import configs
+    cfg = workload_meta(name)
+    if name == "ensemble":
+        fluids = [PlainFluid(int(c), 1000 * seed + k) for k, c in enumerate(configs.replica_sizes(256, seed=seed))]
+        return ([x.copy() for x in fluids for _ in (1, 2, 4)], [PlainLJ()],
+                [0.005 * configs.AR_TAU / f for _ in fluids for f in (1, 2, 4)], cfg)
+    if name == "lj1m":
+        return PlainFluid(64, seed), [PlainLJ()], 0.005 * configs.AR_TAU, cfg
+    if name == "argon864":
+        return PlainFluid(6, seed, T=94.4, L=10.229 * configs.AR_SIGMA), [PlainLJ()], 10 * 1e-15, cfg
+    raise SystemExit(f"the workload {name} needs accusim, which is not importable")
+
+
+def plain_start_engine(systems, forces, dts, rec_cap, tpa, cell_order, cell_scale):
+    """`engine.start_engine` for PlainFluids: the engine under the same rules, its force field filled in here."""
+    import numpy as np
+
+    from devinproj_b200 import configs
+    from devinproj_b200 import engine as E
+    ff = E.ForceField()
+    ff.n_species, ff.lj, ff.lj_cutoff = 1, 1, forces[0].cutoff
+    ff.mass[0], ff.lj_eps[0], ff.lj_sig[0] = configs.AR_MASS / E.MASS, configs.AR_EPS / E.ENERGY, configs.AR_SIGMA / E.LEN
+    rlist, half_skin = (forces[0].cutoff + forces[0].skin) * configs.AR_SIGMA, 0.5 * forces[0].skin * configs.AR_SIGMA
+    maxnb = max(E.estimate_maxnb(s.n, s.box, rlist) for s in systems)
+    if not isinstance(tpa, int):   # the timed autotuner needs accusim's forces: the size rule
+        cells = sum(int(np.prod([max(1, int(b // (rlist * cell_scale))) for b in s.box])) for s in systems)
+        tpa = E.default_tpa(sum(s.n for s in systems), (maxnb - 32) / 1.3, cells)
+    eng = E.Engine([dict(n=s.n, box=s.box / E.LEN, dt=dt / E.TIME, rlist=rlist / E.LEN, half_skin=half_skin / E.LEN)
+                    for s, dt in zip(systems, dts)], ff, maxnb, rec_cap=rec_cap, tpa=tpa, cell_order=cell_order,
+                   cell_scale=cell_scale)
+    E._upload_state(eng, systems)
+    eng.check("engine start")
+    return eng, rlist, half_skin
+
+
 class ClockSampler:
     """nvidia-smi samples of SM clock and throttle reasons while the timed region runs."""
 
@@ -296,6 +380,11 @@ def main():
 
     if args.impl == "reference":
         if rank == 0:
+            try:
+                reference_package()
+            except ImportError as exc:
+                print(json.dumps({"impl": "reference", "unavailable": f"accusim is not installed here: {exc}"}), flush=True)
+                return
             reference_arm(args, full_config(workload_meta(args.workload), args, world))
         return
     if args.experiment:
@@ -312,12 +401,16 @@ def main():
     if world > 1:
         dist.init_process_group("nccl", timeout=timedelta(seconds=120),
                                 device_id=torch.device("cuda", local))
+    from devinproj_b200 import _accusim
     from devinproj_b200.engine import ACC, LEN, VEL, start_engine
+    plain = _accusim.accusim is None
+    if plain:
+        print(f"{_accusim.MISSING}; the LJ workloads run without it", file=sys.stderr)
 
     ensemble = args.workload == "ensemble"
     # the replica ensemble is one workload sharded over the ranks (largest replica first to the least-loaded
     # rank, no collective while stepping); the single-system workloads run one independent copy per rank
-    s, forces, dt, cfg = workload(args.workload, seed=0 if ensemble else rank)
+    s, forces, dt, cfg = (plain_workload if plain else workload)(args.workload, seed=0 if ensemble else rank)
     systems, dts = (s, dt) if isinstance(s, list) else ([s], [dt])
     n_global = sum(x.n for x in systems)
     shard = list(range(len(systems)))
@@ -326,8 +419,8 @@ def main():
         shard = shard_replicas([x.n for x in systems], world)[rank]
         systems, dts = [systems[r] for r in shard], [dts[r] for r in shard]
     rec_cap = max(args.steps // args.record_every + 2, args.drift_steps // args.record_every + 2, 4)
-    eng, rlist, hs = start_engine(systems, forces, dts, rec_cap=rec_cap, tpa=args.tpa, cell_order=args.cell_order,
-                                  cell_scale=args.cell_scale)
+    eng, rlist, hs = (plain_start_engine if plain else start_engine)(
+        systems, forces, dts, rec_cap=rec_cap, tpa=args.tpa, cell_order=args.cell_order, cell_scale=args.cell_scale)
     n = sum(x.n for x in systems)
     pairs_lj, pairs_dsf = eng.count_pairs()
     step_blocks, coop_blocks, slots = eng.launch_info()
