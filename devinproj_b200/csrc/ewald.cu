@@ -227,9 +227,10 @@ __device__ __forceinline__ double ewald_pair(const EwaldPar& P, double r2, doubl
 // through the lanes: 32 rounds of 32 different pairs, after which the forces on the tile are home; those of the block's
 // warps are added in warp order and stored per block, so every sum has a fixed order. Its own tile a warp takes both
 // ways round. Bound by FP64 issue, some 95 operations per round whether few or all of its pairs are inside rcut; the
-// rotation (14 shuffles) hides behind them. 8000 ions: 0.27 ms in 111 parts of a block row (0.29 in 56, 0.34 in 28: a
-// block's share of the triangle shrinks along the rows); the pairs from both sides, a lane per atom (k_ewald_real),
-// 0.55; the whole sum went from 9.75 ms (one thread per atom for all pairs and vectors) to 0.42.
+// rotation (14 shuffles) hides behind them. 8000 ions: 0.29 ms in 111 parts of a block row (0.27 before the pair
+// terms were as exact as now, 0.29 then in 56 parts, 0.34 in 28: a block's share of the triangle shrinks along the rows);
+// the pairs from both sides, a lane per atom (k_ewald_real), 0.55; the whole sum went from 9.75 ms (one thread per atom
+// for all pairs and vectors) to 0.44.
 __global__ void __launch_bounds__(kBlock, 3) k_ewald_tiles(const Packed* __restrict__ pk, int64_t n,
                                                            const __grid_constant__ EwaldPar P,
                                                            Packed* __restrict__ ipart, double* __restrict__ jpart) {

@@ -96,7 +96,7 @@ struct DescPar {
 // (also over the distance, so that a vector term has the roundings of g fc / r d and no more: with a unit vector per
 // neighbour it had one more) of one neighbour per lane, staged in shared memory (species 0 from the front, 1 from the back, each in
 // list order); then lane k adds Gaussian k of every staged neighbour. 8000 ions with 134 neighbours: 457 us when every
-// lane formed every neighbour's distance (with three FP64 divisions), 35 us so, bound by instruction issue (about 12
+// lane formed every neighbour's distance (with three FP64 divisions), 37 us so, bound by instruction issue (about 12
 // per neighbour and warp). A channel's sum adds the same rounded terms in the same order as before, so the BF16
 // invariants are the same bit for bit (their roundings travel through the network).
 __global__ void __launch_bounds__(256) k_descriptors(const double* __restrict__ pos, const int32_t* __restrict__ sp,
