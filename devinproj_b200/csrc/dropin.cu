@@ -423,7 +423,8 @@ __global__ void __launch_bounds__(kBlock) k_list_sparse(const double* __restrict
 // packed FP32 operation; ballots give a home atom's accepted candidates, which its lane then writes. The same lists entry
 // by entry. Boxes with 4 or more cells on every periodic axis. Whole build of the 1,048,576-atom LJ fluid (78 neighbours
 // of 516 candidates): 2.73 ms by a thread per atom in FP64, 1.97 by a warp per atom, 0.71 here, where the lists' 4-byte
-// stores, one sector each, are most of the rest; with the atoms in random order 4.97, 2.35 and 2.51.
+// stores, one sector each, are most of the rest; with the atoms in random order 4.97, 2.35 and 2.51. 80 registers and 36
+// bytes spilled.
 __global__ void __launch_bounds__(kBlock) k_list_cells(const double* __restrict__ pos, const __grid_constant__ GridDev g,
                                                        Screen f, int64_t ncells, const int32_t* __restrict__ start,
                                                        const float4* __restrict__ screen, int maxnb,
@@ -876,8 +877,9 @@ __device__ __forceinline__ void sum_phases(const PairSplit& sp, double (&v)[4]) 
 // around each pair and three rounding instructions per minimum image: 0.67). Three gathers and the next list entries
 // in flight at 64 registers; more of either loses the occupancy that hides the FP64 chains (0.32 to 0.44 measured). An
 // 864-atom box: 52 -> 5.8 us; 256 atoms without a list: 92 -> 6.8. PACKED gathers one 256-bit record per neighbour,
-// otherwise from the caller's arrays (pack_gathers; the entry point without a work buffer). ONE: a single species, its constants in registers; else the species-pair tables
-// are staged in shared memory (a kernel parameter indexed per thread serialises).
+// otherwise from the caller's arrays (pack_gathers; the entry point without a work buffer). The list variants spill 8
+// (ONE) to 24 bytes at the 64 registers that four blocks per SM leave. ONE: a single species, its constants in registers;
+// else the species-pair tables are staged in shared memory (a kernel parameter indexed per thread serialises).
 template <bool DENSE, bool PACKED, bool ONE>
 __global__ void __launch_bounds__(kBlock, 4) k_lj64(const double* __restrict__ pos, const int32_t* __restrict__ sp,
                                                   const Packed* __restrict__ pk, int64_t n, ImageBox box,
